@@ -101,6 +101,19 @@ void setup_boundary(BoundaryDev& b, const wq3d_boundary_desc& d, double R) {
         b.loss.rl_att = b.loss.p[2] * ATT_CONVERT;
         b.loss.rl_shr = 1500.0 * b.loss.p[3];
         b.loss.rl_satt = b.loss.p[4] * ATT_CONVERT;
+        LossDev& L = b.loss;
+        L.rl_fast = 1;
+        for (double v : {L.rl_den, L.rl_spd, L.rl_att, L.rl_shr, L.rl_satt})
+            if (!(v == 0.0 || (std::abs(v) > 1e-30 && std::abs(v) < 1e30))) L.rl_fast = 0;
+        L.rl_shear_const = L.rl_shr == 0.0;
+        if (L.rl_shear_const) {
+            cplx cos2, add;
+            rl_shear(L, 1.0, &cos2, &add);
+            L.rl_cos2[0] = cos2.re;
+            L.rl_cos2[1] = cos2.im;
+            L.rl_add[0] = add.re;
+            L.rl_add[1] = add.im;
+        }
     }
 }
 
@@ -175,14 +188,52 @@ int make_grid(wq3d_ocean* o, const wq3d_grid_desc& d, int max_dims, GridDev* hg,
         hg->edge[k] = d.edge_limit[k] ? 1 : 0;
     }
     if (!d.data) return fail(WQ3D_ERR_INVALID, "grid data missing");
-    hg->all_linear = 1;
-    for (int k = 0; k < d.ndim; ++k)
-        if (hg->interp[k] != WQ3D_INTERP_LINEAR) hg->all_linear = 0;
-    hg->pchip0 = hg->interp[0] == WQ3D_INTERP_PCHIP;
-    for (int k = 1; k < d.ndim; ++k)
-        if (hg->interp[k] != WQ3D_INTERP_LINEAR) hg->pchip0 = 0;
     o->store.emplace_back(d.data, d.data + total);
     hg->data = o->store.back().data();
+    /* The unrolled device evaluation: its tables, and whether every
+     * denominator and dividend stays within quot()'s range.  Magnitudes up
+     * to 1e18 that differ by 1e-18 or more keep all quotients far from the
+     * ends of the exponent range; an earth's grid is well inside. */
+    hg->unrolled = GRID_LINEAR;
+    if (hg->interp[0] == WQ3D_INTERP_PCHIP) hg->unrolled = GRID_PCHIP0;
+    else if (hg->interp[0] != WQ3D_INTERP_LINEAR) hg->unrolled = GRID_GENERAL;
+    for (int k = 1; k < d.ndim; ++k)
+        if (hg->interp[k] != WQ3D_INTERP_LINEAR) hg->unrolled = GRID_GENERAL;
+    bool ok = true;
+    auto size_ok = [](double v) { return v == 0.0 || (std::abs(v) > 1e-18 && std::abs(v) < 1e18); };
+    auto step_ok = [&](double v) { return v != 0.0 && size_ok(v) && divisor_ok(v); };
+    for (size_t i = 0; i < total; ++i) ok = ok && (std::isnan(hg->data[i]) || size_ok(hg->data[i]));
+    std::vector<double> lin[3], pch;
+    for (int k = 0; k < d.ndim; ++k) {
+        AxisDev& ax = hg->ax[k];
+        ax.x0 = ax.x[0];
+        ax.xl = ax.x[ax.n - 1];
+        ax.inc0 = ax.inc[0];
+        ax.rinc0 = 1.0 / ax.inc0;
+        ax.top_bit = 1;
+        while (2 * ax.top_bit <= ax.n - 1) ax.top_bit *= 2;
+        lin[k].resize(4 * (size_t)ax.n);
+        for (int i = 0; i < ax.n; ++i) {
+            const double h = axis_inc(ax, i);
+            ok = ok && size_ok(ax.x[i]) && step_ok(h);
+            lin[k][4 * i] = ax.x[i];
+            lin[k][4 * i + 1] = h;
+            lin[k][4 * i + 2] = 1.0 / h;
+        }
+    }
+    if (hg->unrolled == GRID_PCHIP0) {
+        const AxisDev& ax = hg->ax[0];
+        pch.resize(16 * (size_t)ax.n);
+        for (int i = 0; i < ax.n; ++i) {
+            const double h0 = axis_inc(ax, (long)i - 1), h1 = axis_inc(ax, i), h2 = axis_inc(ax, (long)i + 1);
+            const double h1_2 = h1 * h1, h1_3 = h1_2 * h1, ha = h1 + h2, hb = h1 + h0;
+            ok = ok && divisor_ok(h1_2) && divisor_ok(h1_3) && step_ok(ha) && step_ok(hb);
+            const double row[16] = {ax.x[i], h1, 1.0 / h1, h0, 1.0 / h0, h2, 1.0 / h2, h1_2,
+                                    1.0 / h1_2, h1_3, 1.0 / h1_3, ha, 1.0 / ha, hb, 1.0 / hb, 0.0};
+            std::copy(row, row + 16, &pch[16 * (size_t)i]);
+        }
+    }
+    if (!ok) hg->unrolled = GRID_GENERAL;
     *dg = *hg;
     auto up = [&](const double* src, size_t n, const double** out) -> int {
         void* p = nullptr;
@@ -196,7 +247,9 @@ int make_grid(wq3d_ocean* o, const wq3d_grid_desc& d, int max_dims, GridDev* hg,
     for (int k = 0; k < d.ndim && !rc; ++k) {
         rc = up(hg->ax[k].x, hg->ax[k].n, &dg->ax[k].x);
         if (!rc) rc = up(hg->ax[k].inc, hg->ax[k].n, &dg->ax[k].inc);
+        if (!rc && hg->unrolled != GRID_GENERAL) rc = up(lin[k].data(), lin[k].size(), &dg->ax[k].lin);
     }
+    if (!rc && hg->unrolled == GRID_PCHIP0) rc = up(pch.data(), pch.size(), &dg->ax[0].pch);
     if (!rc) rc = up(hg->data, total, &dg->data);
     return rc;
 }

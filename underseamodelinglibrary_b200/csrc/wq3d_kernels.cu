@@ -91,7 +91,7 @@ __device__ __forceinline__ void profile_at(const QueueDev& q, const double* pos,
 __device__ __forceinline__ void update1(const QueueDev& q, RayS& y) {
     profile_at(q, y.pos, &y.c, y.sg);
     double st;
-    ray_derivs(y.c, y.sg[0], y.sg[1], y.sg[2], y.pos, y.nd, y.pg, y.ng, &st);
+    ray_derivs<!WQ3D_WITH_GRID>(y.c, y.sg[0], y.sg[1], y.sg[2], y.pos, y.nd, y.pg, y.ng, &st);
 }
 
 /* wave_front::update of the FP32 propagation form (no distance terms) */
@@ -219,7 +219,7 @@ __device__ __forceinline__ void update_main(const QueueDev& q, const FrontPtrs& 
                                             const FrontPtrs* src) {
     profile_at(q, y.pos, &y.c, y.sg);
     double st;
-    ray_derivs(y.c, y.sg[0], y.sg[1], y.sg[2], y.pos, y.nd, y.pg, y.ng, &st);
+    ray_derivs<!WQ3D_WITH_GRID>(y.c, y.sg[0], y.sg[1], y.sg[2], y.pos, y.nd, y.pg, y.ng, &st);
     copy_ray(f, r, y);
     f.cpa[0][r] = y.pos[0];
     f.cpa[1][r] = y.pos[1];
@@ -1089,7 +1089,7 @@ __device__ __forceinline__ void advance_body(const QueueDev& q, int k) {
         st = sin(y3.pos[1]);
     } else {
         profile_at(q, y3.pos, &y3.c, y3.sg);
-        ray_derivs(y3.c, y3.sg[0], y3.sg[1], y3.sg[2], y3.pos, y3.nd, y3.pg, y3.ng, &st);
+        ray_derivs<!WQ3D_WITH_GRID>(y3.c, y3.sg[0], y3.sg[1], y3.sg[2], y3.pos, y3.nd, y3.pg, y3.ng, &st);
     }
     const uint8_t f_next = reflect_decision(q, y3.pos, y2.nd);
     /* the per-step finiteness check: a NaN or Inf in the environment (a
