@@ -256,6 +256,171 @@ int make_grid(wq3d_ocean* o, const wq3d_grid_desc& d, int max_dims, GridDev* hg,
 
 }  // namespace
 
+namespace {
+
+/* the CPA search's view of the targets (QueueDev::clusters, cpa_tgt,
+ * cpa_index, tgt_box) */
+struct CpaTargets {
+    std::vector<TgtCluster> clusters;
+    std::vector<double> tgt;
+    std::vector<uint32_t> index;
+    double box[6] = {0, 0, 0, 0, 0, 0};
+};
+
+/* the clusters of the targets in the given order, and the sum of their
+ * extents in metres */
+double make_clusters(const std::vector<double>& r, const std::vector<double>& th, const std::vector<double>& ph,
+                     const std::vector<double>& sn, const std::vector<uint8_t>& branch,
+                     const std::vector<uint32_t>& order, std::vector<TgtCluster>* out) {
+    out->clear();
+    double total = 0.0;
+    for (size_t b = 0; b < order.size(); b += 32) {
+        const size_t e = std::min(order.size(), b + 32);
+        double lo[4], hi[4];
+        for (size_t j = b; j < e; ++j) {
+            const uint32_t t = order[j];
+            const double v[4] = {r[t], th[t], ph[t], r[t] * sn[t]};
+            for (int k = 0; k < 4; ++k) {
+                /* a NaN stays, and makes the cluster's bounds NaN */
+                if (j == b || !(v[k] >= lo[k])) lo[k] = v[k];
+                if (j == b || !(v[k] <= hi[k])) hi[k] = v[k];
+            }
+        }
+        TgtCluster c{};
+        for (size_t j = b; j < e; ++j) c.branch |= branch[order[j]];
+        double mid[4], half[4];
+        for (int k = 0; k < 4; ++k) {
+            mid[k] = 0.5 * (lo[k] + hi[k]);
+            half[k] = std::max(hi[k] - mid[k], mid[k] - lo[k]) * 1.000001;
+        }
+        c.R = mid[0];
+        c.T = mid[1];
+        c.P = mid[2];
+        c.RS = mid[3];
+        c.dR = (float)half[0];
+        c.dT = (float)half[1];
+        c.dP = (float)half[2];
+        c.dRS = (float)half[3];
+        total += half[0] + std::abs(mid[0]) * half[1] + std::abs(mid[3]) * half[2];
+        out->push_back(c);
+    }
+    return total;
+}
+
+/* Clusters of 32 consecutive targets, in the caller's order or along a
+ * Morton curve, whichever has the smaller extents: a range x depth table's
+ * columns are already compact (1.5 of 32 clusters survive a warp's bounds on
+ * the sloped workload, 3 along the curve), random targets are not (27 of 128
+ * on the reverberation workload, 126 in their own order). */
+void cpa_targets(const std::vector<double>& r, const std::vector<double>& th, const std::vector<double>& ph,
+                 const std::vector<double>& sn, const std::vector<uint8_t>& branch, CpaTargets* o) {
+    const size_t nt = r.size();
+    o->index.resize(nt);
+    for (size_t t = 0; t < nt; ++t) o->index[t] = (uint32_t)t;
+    double lo[3], hi[3];
+    for (size_t t = 0; t < nt; ++t) {
+        const double v[3] = {r[t], th[t], ph[t]};
+        for (int k = 0; k < 3; ++k) {
+            if (t == 0 || !(v[k] >= lo[k])) lo[k] = v[k];
+            if (t == 0 || !(v[k] <= hi[k])) hi[k] = v[k];
+        }
+    }
+    for (int k = 0; k < 3 && nt; ++k) {
+        o->box[2 * k] = lo[k];
+        o->box[2 * k + 1] = hi[k];
+    }
+    const double own = make_clusters(r, th, ph, sn, branch, o->index, &o->clusters);
+    if (nt > 32) {
+        const double size = std::max({hi[0] - lo[0], hi[0] * (hi[1] - lo[1]), hi[0] * (hi[2] - lo[2])});
+        if (size > 0.0 && size < 1e30) {
+            std::vector<std::pair<uint64_t, uint32_t>> key(nt);
+            for (size_t t = 0; t < nt; ++t) {
+                const double x[3] = {r[t] - lo[0], hi[0] * (th[t] - lo[1]), hi[0] * sn[t] * (ph[t] - lo[2])};
+                uint64_t m = 0;
+                for (int k = 0; k < 3; ++k) {
+                    const uint32_t c = (uint32_t)std::min(1023.0, std::max(0.0, 1023.0 * x[k] / size));
+                    for (int b = 0; b < 10; ++b) m |= (uint64_t)((c >> b) & 1u) << (3 * b + k);
+                }
+                key[t] = {m, (uint32_t)t};
+            }
+            std::sort(key.begin(), key.end());
+            std::vector<uint32_t> order(nt);
+            for (size_t t = 0; t < nt; ++t) order[t] = key[t].second;
+            std::vector<TgtCluster> cl;
+            if (make_clusters(r, th, ph, sn, branch, order, &cl) < own) {
+                o->index.swap(order);
+                o->clusters.swap(cl);
+            }
+        }
+    }
+    o->tgt.resize(4 * nt);
+    for (size_t j = 0; j < nt; ++j) {
+        const uint32_t t = o->index[j];
+        o->tgt[4 * j] = r[t];
+        o->tgt[4 * j + 1] = th[t];
+        o->tgt[4 * j + 2] = ph[t];
+        o->tgt[4 * j + 3] = sn[t];
+    }
+}
+
+/* The patches of rays that CPA warps take: bands of 32, 16, 8, 4, 2 or 1
+ * D/E rows cut along AZ.  A band's shape keeps the angular extents of its
+ * patches smallest: its D/E span against half the AZ span, times the cosine
+ * of its D/E angle (a fan's AZ rays close up towards the vertical, where a
+ * tangent-spaced fan's D/E rays open).  Targets kept per ray, against 32 x 1
+ * rays throughout: 30 for 36 of 1024 (sloped workload, step 100), 52 for 123
+ * of 4096 (reverberation workload), 10 for 34 of 100 (Munk workload).  The
+ * steep bands, which keep the most, come first. */
+constexpr int CPA_PARTS = 8;
+
+/* the most patches that a fan of this size can have: a band of r rows has
+ * at most naz r / 32 + 1 */
+size_t cpa_patch_limit(size_t nde, size_t naz) { return CPA_PARTS * (naz * (nde + 31) / 32 + nde + 1); }
+
+void cpa_patches(const std::vector<double>& de, const std::vector<double>& az, size_t nt,
+                 std::vector<CpaPatch>* out) {
+    const int nde = (int)de.size(), naz = (int)az.size();
+    out->clear();
+    if (nde < 3 || naz < 3) return;
+    const double da = std::abs(az.back() - az.front()) / (double)(naz - 1);
+    struct Band {
+        int de, shift;
+        double steep;
+    };
+    std::vector<Band> bands;
+    size_t patches = 0;
+    for (int d = 0; d < nde;) {
+        int best = 0;
+        double least = 0.0;
+        for (int s = 0; s <= 5; ++s) {
+            const int e = std::min(nde - 1, d + (32 >> s) - 1);
+            double c = 0.0;
+            for (int j = d; j <= e; ++j) c = std::max(c, std::abs(std::cos(to_radians(de[j]))));
+            const double span_de = std::abs(de[e] - de[d]) + 0.5 * std::abs(de[std::min(nde - 1, d + 1)] - de[d]);
+            const double span = std::max(span_de, 0.5 * (double)((1 << s) - 1) * da * c);
+            if (s == 0 || span < least) {
+                best = s;
+                least = span;
+            }
+        }
+        bands.push_back({d, best, std::abs(de[d])});
+        patches += (naz + (1 << best) - 1) >> best;
+        d += 32 >> best;
+    }
+    std::stable_sort(bands.begin(), bands.end(), [](const Band& x, const Band& y) { return x.steep > y.steep; });
+    /* A fan with fewer patches than the GPU has room for (592 schedulers,
+     * four warps each) splits the clusters, four a share at least. */
+    const size_t ncl = (nt + 31) / 32;
+    const size_t parts = std::max<size_t>(
+        1, std::min({(size_t)CPA_PARTS, 4 * 592 / std::max<size_t>(patches, 1), ncl / 4}));
+    for (const Band& b : bands)
+        for (size_t p = 0; p < parts; ++p)
+            for (int a = 0; a < naz; a += 1 << b.shift)
+                out->push_back({b.de, (int16_t)a, (uint8_t)b.shift, (uint8_t)p, (uint8_t)parts, {0, 0, 0}});
+}
+
+}  // namespace
+
 /* The reflection-schedule plan learnt per queue shape (fan, targets,
  * frequencies, kernel build, chunk length), shared by every queue of the
  * process.  A run is cut into buckets of TUNE_BUCKET steps, since which
@@ -353,8 +518,9 @@ struct wq3d_queue {
     /* per result set: chunk base step, chunk times, counters read back
      * (n_rec, n_refl, err, -, work lists, n_done, -, n_verb); d_counts also
      * holds the bottom work lists (9, 10), the adjoint's mark and entry
-     * count (11, 12), the three candidate counts (13-15) and the three
-     * shadow sets' inline slot counts (16-18) */
+     * count (11, 12), the three candidate counts (13-15), the three
+     * shadow sets' inline slot counts (16-18) and the CPA search's item
+     * counts (20, 21) */
     int64_t* h_base[2] = {nullptr, nullptr};
     double* h_times[2] = {nullptr, nullptr};
     uint32_t* h_counts[2] = {nullptr, nullptr};
@@ -672,14 +838,14 @@ struct wq3d_queue {
         /* eigenray candidates grow with the fan: one block per SM for small
          * fans, up to EIG_BLOCKS */
         const int eig_blocks = std::min(EIG_BLOCKS, std::max(148, (n + 255) / 256));
+        /* and so do the items of its CPA search */
+        const int item_blocks = std::min(CPA_ITEM_BLOCKS, std::max(148, (n + 255) / 256));
         if (timing) tail = false;
         auto cpa_launch = [&](int k, cudaStream_t st) {
-            const dim3 cgrid(((h.nde + CPA_PATCH_DE - 1) / CPA_PATCH_DE) * ((h.naz + CPA_PATCH_AZ - 1) / CPA_PATCH_AZ),
-                             (h.nt + CPA_F32_TARGETS - 1) / CPA_F32_TARGETS);
-            if (h.precision != WQ3D_FP64)
-                k_cpa_f32<<<cgrid, CPA_THREADS, 0, st>>>(d, k);
-            else
-                k_cpa<<<cgrid, CPA_THREADS, 0, st>>>(d, k);
+            const int cgrid = std::max(1, (h.n_patch + CPA_WARPS - 1) / CPA_WARPS);
+            k_cpa<<<cgrid, 32 * CPA_WARPS, 0, st>>>(d, k);
+            k_cpa_items<<<item_blocks, 128, 0, st>>>(d, k);
+            launches += 2;
         };
         auto eig_launch = [&](int k, cudaStream_t st) {
             k_eigenray<<<eig_blocks, 128, 0, st>>>(d, k);
@@ -722,7 +888,6 @@ struct wq3d_queue {
                 cudaEventRecord(ev[2], stream);
                 if (h.nt > 0) {
                     cpa_launch(k, stream);
-                    launches += 1;
                     cudaEventRecord(ev[3], stream);
                     eig_launch(k, stream);
                 } else {
@@ -779,7 +944,6 @@ struct wq3d_queue {
             cudaStreamWaitEvent(stream, adv_ev[k], 0);
             if (h.nt > 0) {
                 cpa_launch(k, stream);
-                launches += 1;
                 cudaEventRecord(cpa_ev[k], stream);
                 cudaStreamWaitEvent(eig, cpa_ev[k], 0);
                 eig_launch(k, eig);
@@ -1549,6 +1713,13 @@ int wq3d_queue_create(const wq3d_ocean* ocean, const wq3d_queue_desc* d, wq3d_qu
         const double tlng = to_degrees(tp[t]);
         tbranch[t] = (std::abs(slat - tlat) < 1e-4 && std::abs(slng - tlng) < 1e-4) ? 1 : 0;
     }
+    CpaTargets cpa;
+    cpa_targets(tr, tt, tp, tsin, tbranch, &cpa);
+    std::copy(cpa.box, cpa.box + 6, h.tgt_box);
+    std::vector<CpaPatch> patches;
+    if (nt) cpa_patches(de, az, nt, &patches);
+    h.n_patch = (int)patches.size();
+    patches.resize(nt ? cpa_patch_limit(nde, naz) : 0); /* a reused queue keeps its buffer */
     /* spreading normalisation (spreading_hybrid_gaussian.cc:28-59,
      * spreading_ray.cc:26-45) */
     std::vector<double> norm_de(nde, 0.0), norm_az(n, 0.0), init_area(n, 0.0);
@@ -1585,7 +1756,8 @@ int wq3d_queue_create(const wq3d_ocean* ocean, const wq3d_queue_desc* d, wq3d_qu
         (rc = q->upload(&h.tgt[2], tp)) || (rc = q->upload(&h.tgt_sin, tsin)) ||
         (rc = q->upload(&h.tgt_R2, tR2)) || (rc = q->upload(&h.tgt_2R, t2R)) ||
         (rc = q->upload(&h.tgt_spread2, tspread)) || (rc = q->upload(&h.tgt_c, tc)) ||
-        (rc = q->upload(&h.de_branch, tbranch)) || (rc = q->upload(&h.norm_de, norm_de)) ||
+        (rc = q->upload(&h.patches, patches)) || (rc = q->upload(&h.clusters, cpa.clusters)) || (rc = q->upload(&h.cpa_tgt, cpa.tgt)) ||
+        (rc = q->upload(&h.cpa_index, cpa.index)) || (rc = q->upload(&h.de_branch, tbranch)) || (rc = q->upload(&h.norm_de, norm_de)) ||
         (rc = q->upload(&h.norm_az, norm_az)) || (rc = q->upload(&h.init_area, init_area)))
         return cleanup(rc);
 
@@ -1650,10 +1822,14 @@ int wq3d_queue_create(const wq3d_ocean* ocean, const wq3d_queue_desc* d, wq3d_qu
         uint32_t* cand = nullptr;
         if ((rc = q->alloc(&cand, 2 * CAND_LISTS * (size_t)h.cap_cand))) return cleanup(rc);
         h.cand = cand;
+        /* items of the CPA search: a few per patch at most on the measured
+         * workloads; k_cpa decides those that find no room */
+        h.cap_item = (uint32_t)std::max<size_t>(4096, std::min<size_t>((size_t)1 << 20, 8 * patches.size()));
+        if ((rc = q->alloc(&h.items, h.cap_item))) return cleanup(rc);
         if ((rc = q->alloc(&h.rec, h.cap_rec)) || (rc = q->alloc(&h.rec_inten, (size_t)h.cap_rec * nf)) ||
             (rc = q->alloc(&h.rec_phase, (size_t)h.cap_rec * nf)) || (rc = q->alloc(&h.refl, h.cap_refl)))
             return cleanup(rc);
-        if ((rc = q->alloc(&q->d_counts, 20)) || (rc = q->alloc(&q->d_base, 1)) ||
+        if ((rc = q->alloc(&q->d_counts, 24)) || (rc = q->alloc(&q->d_base, 1)) ||
             (rc = q->alloc(&q->d_times, (size_t)q->chunk + 1)))
             return cleanup(rc);
     }
@@ -1668,6 +1844,7 @@ int wq3d_queue_create(const wq3d_ocean* ocean, const wq3d_queue_desc* d, wq3d_qu
     h.n_done = q->d_counts + 6;
     h.n_verb = q->d_counts + 8;
     h.n_slot = q->d_counts + 16; /* one per shadow set: 16, 17, 18 */
+    h.n_item = q->d_counts + 20; /* by step parity: 20, 21 */
     h.want_verbs = 0;
     h.verb_threshold = 1e-30; /* wave_thresholds.h:40 */
     if (!reuse) {
@@ -1697,7 +1874,7 @@ int wq3d_queue_create(const wq3d_ocean* ocean, const wq3d_queue_desc* d, wq3d_qu
             q->h_times[s] = reinterpret_cast<double*>(b + 128);
         }
     }
-    if (cudaMemset(q->d_counts, 0, 20 * sizeof(uint32_t)) != cudaSuccess)
+    if (cudaMemset(q->d_counts, 0, 24 * sizeof(uint32_t)) != cudaSuccess)
         return cleanup(fail(WQ3D_ERR_CUDA, "cudaMemset failed"));
 
     /* wave_queue ctor: init_wave, update, init_wavefronts */

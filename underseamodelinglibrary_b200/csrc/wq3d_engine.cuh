@@ -107,6 +107,23 @@ struct AdjRec {
 };
 enum : int32_t { ADJ_VALID = 1, ADJ_CELL_OVERFLOW = 2 };
 
+/* the work of a CPA warp: (32 >> shift) D/E x (1 << shift) AZ rays from
+ * (de, az), against one of "parts" equal shares of the target clusters */
+struct CpaPatch {
+    int32_t de;
+    int16_t az;
+    uint8_t shift, part, parts, pad[3];
+};
+
+/* 32 targets of the CPA search: the middle of their ranges of rho, theta,
+ * phi and rho sin(theta), and the half-widths (rounded up) */
+struct TgtCluster {
+    double R, T, P, RS;
+    float dR, dT, dP, dRS;
+    int32_t branch; /* holds a target with QueueDev::de_branch set */
+    int32_t pad;
+};
+
 struct FrontPtrs {
     double* pos[3];
     double* pg[3];
@@ -160,6 +177,16 @@ struct QueueDev {
     const double* tgt_spread2;   /* [nt][nf] (2 pi c_target / f)^2 */
     const double* tgt_c;         /* sound speed at each target */
     const uint8_t* de_branch;
+    /* the CPA search's targets, in clusters of 32 that lie near one another */
+    const TgtCluster* clusters;
+    const double* cpa_tgt;       /* [nt][4] rho, theta, phi, sin(theta) */
+    const uint32_t* cpa_index;   /* [nt] index of each in the arrays above */
+    double tgt_box[6];           /* least and largest rho, theta, phi   */
+    const CpaPatch* patches;     /* [n_patch] work of each CPA warp     */
+    int n_patch;
+    uint4* items;                /* [cap_item] (patch, target, rays) left by k_cpa */
+    uint32_t* n_item;            /* [2] by step parity                        */
+    uint32_t cap_item;
     /* spreading normalisation */
     const double* norm_de;
     const double* norm_az;
@@ -256,7 +283,8 @@ WQ3D_DECLARE_STEP_KERNELS
 __global__ void k_volume(__grid_constant__ const QueueDev q, int k);
 __global__ void k_commit(__grid_constant__ const QueueDev q, int k);
 __global__ void k_cpa(__grid_constant__ const QueueDev q, int k);
-__global__ void k_cpa_f32(__grid_constant__ const QueueDev q, int k);
+__global__ void k_cpa_items(__grid_constant__ const QueueDev q, int k);
+constexpr int CPA_ITEM_BLOCKS = 4 * 148; /* four warps each */
 /* k_eigenray blocks (4 warps each, one candidate per warp pair at a
  * time): four per SM, so a step's candidates usually all run at once */
 constexpr int EIG_BLOCKS = 4 * 148;
@@ -316,9 +344,6 @@ __global__ void k_adj_reverse(AdjSweep a, __grid_constant__ const QueueDev q);
 __global__ void k_adj_startup(AdjSweep a, __grid_constant__ const QueueDev q);
 
 
-constexpr int CPA_THREADS = 128;     /* rays per CPA block            */
-constexpr int CPA_F32_TARGETS = 256; /* targets per FP32C CPA tile    */
-constexpr int CPA_PATCH_AZ = 8;      /* FP32C CPA block: 16 D/E x 8 AZ rays */
-constexpr int CPA_PATCH_DE = CPA_THREADS / CPA_PATCH_AZ;
+constexpr int CPA_WARPS = 4; /* independent warps per CPA block */
 
 }  // namespace wq3d

@@ -19,11 +19,11 @@
  *   k_commit    writes the reflected rays' slots and the caustic and vertex
  *               counts into the fronts, on the eigenray stream.
  *   k_cpa       closest-point-of-approach test (detect_eigenrays +
- *               is_closest_ray) over patches of neighbouring rays x tiles
- *               of targets, with distance2 recomputed from per-front terms
- *               and targets no ray of a patch can keep dropped first;
- *               k_cpa_f32 screens each pair in FP32 before the FP64
- *               comparisons.
+ *               is_closest_ray), a warp of neighbouring rays against
+ *               clusters of targets, with distance2 recomputed from
+ *               per-front terms and the targets that no ray of the warp
+ *               can keep dropped by FP32 bounds; k_cpa_items decides the
+ *               rest in FP64.
  *   k_eigenray  one warp per CPA found: build_eigenray, compute_offsets,
  *               hybrid Gaussian or classic spreading, target angles.
  *
@@ -44,6 +44,7 @@
 #define WQ3D_STEP_KERNELS_ONLY 0
 #endif
 #include <cuda_runtime.h>
+#include <stddef.h>
 #include <stdint.h>
 
 #include "wq3d_engine.cuh"
@@ -1316,43 +1317,40 @@ __device__ __forceinline__ int wrap_az(const QueueDev& q, int az, int na) {
     return a;
 }
 
-/* is_closest_ray (wave_queue.cc:411-488); also fills the cube */
-__device__ bool is_closest(const QueueDev& q, const FrontPtrs& V, const FrontPtrs& C,
-                           const FrontPtrs& X, const TgtS& t, bool de_branch, int de,
-                           int az, double center, double cube[3][3][3]) {
+/* is_closest_ray (wave_queue.cc:411-488).  The reference tests each
+ * neighbour on the curr, next and prev fronts in turn and stops at the first
+ * that fails; the order does not matter, so the curr front goes first, where
+ * most pairs fail, with the loads of all eight neighbours in flight at once
+ * (one after another with an early exit, 32 pairs took 12,000 cycles). */
+__device__ __forceinline__ bool is_closest(const QueueDev& q, const FrontPtrs& V, const FrontPtrs& C,
+                                           const FrontPtrs& X, const TgtS& t, bool de_branch, int de,
+                                           int az, double center) {
     const int max_az = q.naz - 1;
-    for (int nd_ = 0; nd_ < 3; ++nd_) {
-        for (int na = 0; na < 3; ++na) {
-            if (nd_ == 1 && na == 1) continue;
-            const int d = de + nd_ - 1;
-            const int a = wrap_az(q, az, na);
-            const int i = d * q.naz + a;
-            cube[0][nd_][na] = d2_at(V, i, t);
-            cube[1][nd_][na] = d2_at(C, i, t);
-            cube[2][nd_][na] = d2_at(X, i, t);
-            if (a == 0 && !q.az_boundary) continue;
-            if (a == max_az) continue;
-            if (de_branch) {
-                if (C.on_edge[i]) continue;
-            } else {
-                if (nd_ != 1 && C.on_edge[i]) continue;
-            }
-            if (nd_ == 2 || na == 2) {
-                if (de_branch) {
-                    if (az == 0) {
-                        if (cube[1][nd_][na] < center) return false;
-                    } else {
-                        return false;
-                    }
-                } else {
-                    if (cube[1][nd_][na] <= center) return false;
-                }
-            } else {
-                if (cube[1][nd_][na] < center) return false;
-            }
-            if (cube[2][nd_][na] <= center) return false;
-            if (cube[0][nd_][na] < center) return false;
-        }
+    double d[9];
+    unsigned compared = 0; /* neighbours that take part */
+#pragma unroll
+    for (int nb = 0; nb < 9; ++nb) {
+        if (nb == 4) continue;
+        const int a = wrap_az(q, az, nb % 3);
+        const int i = (de + nb / 3 - 1) * q.naz + a;
+        const bool edge = C.on_edge[i] != 0;
+        d[nb] = d2_at(C, i, t);
+        const bool skip = (a == 0 && !q.az_boundary) || a == max_az || ((de_branch || nb / 3 != 1) && edge);
+        compared |= skip ? 0u : 1u << nb;
+    }
+    bool fails = false;
+#pragma unroll
+    for (int nb = 0; nb < 9; ++nb) {
+        if (nb == 4) continue;
+        const bool after = nb / 3 == 2 || nb % 3 == 2;
+        const bool nearer = d[nb] < center || (after && !de_branch && d[nb] == center) || (after && de_branch && az != 0);
+        fails |= nearer && ((compared >> nb) & 1u);
+    }
+    if (fails) return false;
+    for (int nb = 0; nb < 9; ++nb) {
+        if (!((compared >> nb) & 1u)) continue;
+        const int i = (de + nb / 3 - 1) * q.naz + wrap_az(q, az, nb % 3);
+        if (d2_at(X, i, t) <= center || d2_at(V, i, t) < center) return false;
     }
     return true;
 }
@@ -1360,338 +1358,430 @@ __device__ bool is_closest(const QueueDev& q, const FrontPtrs& V, const FrontPtr
 }  // namespace
 
 /* ------------------------------------------------------------------ */
-/* CPA search over ray patches, with an FP32 screen in the FP32C form     */
+/* CPA search: a warp of neighbouring rays against clusters of targets   */
 /* ------------------------------------------------------------------ */
-/* The comparisons that reject almost every (ray, target) pair -- "next <=
- * curr" and "prev < curr" on distance2 (wave_queue.cc:386-393) -- are
- * decided from the sign of a distance2 difference.  With coordinates
- * relative to a reference ray of the block (r = rho - rho0, x = theta -
- * theta0, y = phi - phi0; target Rr, X, Y likewise) the reference's
- * distance2 is, in exact arithmetic,
+/* A pair (ray, target) is kept when the ray is nearest the target on the
+ * curr front among its prev and next selves (wave_queue.cc:386-393) and its
+ * neighbours (is_closest_ray).  Each comparison is the sign of a difference
+ * of two distance2 values.  With coordinates relative to a reference ray (r
+ * = rho - rho0, x = theta - theta0, y = phi - phi0; target Rr, X, Y
+ * likewise) the reference's distance2 is, in exact arithmetic,
  *     Rr^2 + sum_k w_k(target) q_k(ray)
- *     q = (r^2, r, rho x^2, rho x, rho, rho s y^2, rho s y, rho s)
- *     w = (1, -2 Rr, R, -2 R X, R X^2, R S, -2 R S Y, R S Y^2)
- * (s = sin theta, S = sin Theta), so a difference of two fronts is
- * sum_k w_k dq_k: the per-ray feature differences dq_k are formed once in
- * FP64, and each pair costs 8 FP32 FMAs per comparison.  A comparison is
- * accepted in FP32 only when the difference exceeds 32 u sum_k W_k |dq_k|
- * (W_k = largest |w_k| of the target tile, u = 2^-24; the FP32 evaluation
- * error is below 12 u of that sum) plus max(1 m^2, 4e-15 (rho^2 + R^2))
- * for the rounding of the reference's FP64 expression on the two fronts
- * (each within 5 x 2^-53 (rho^2 + R^2), 0.05 m^2 at earth radius).  The
- * screen only rejects; every pair it does not reject is queued per warp and
- * finished with the FP64 comparisons, 32 at a time so the lanes stay
- * converged.  Hence the eigenrays equal the FP64 form's, which runs the
- * same patch search with every surviving pair going to those comparisons
- * (k_cpa).
+ *     q = (r^2, rho, rho x^2, rho x, rho s y^2, rho s y, rho s)
+ *     w = (1, R X^2 - 2 Rr, R, -2 R X, R S, -2 R S Y, R S Y^2)
+ * (s = sin theta, S = sin Theta), so the difference of a point (the ray on
+ * another front, or a neighbour) from the ray on the curr front is sum_k
+ * w_k dq_k, with seven features dq_k per ray that do not depend on the
+ * target.
  *
- * A block holds a patch of CPA_PATCH_DE x CPA_PATCH_AZ neighbouring rays,
- * whose positions and directions are close, so for a given target the
- * screen's value sum_k w_k dq_k varies little across the patch.  Before
- * the per-ray loop, each target is tested once for the whole patch: with
- * lo_k <= dq_k <= hi_k over the patch's rays, sum_k max(w_k lo_k, w_k hi_k)
- * (exact products of FP32 values, summed in FP64) bounds every ray's exact
- * value; adding the FP32 evaluation error (8 u sum W_k M_k, M_k = max
- * |dq_k|) and the largest guard of the patch (33 u sum W_k M_k + c0), a
- * negative bound means every ray of the patch would reject the target, so
- * it is dropped before the loop.  Only the targets that survive for the
- * "next" and the "prev" comparison reach the per-ray loop. */
+ * One warp holds a patch of 32 neighbouring rays (QueueDev::patches) and
+ * works without block barriers.  Six differences can each reject a target
+ * for every ray of the patch, when an upper bound of theirs is negative:
+ * the AZ neighbours' (next, prev), the next and prev fronts', and the D/E
+ * neighbours'.  They are bounded
+ *   per cluster  of 32 targets near one another, one lane each, from the
+ *                patch's feature ranges and the cluster's centre and
+ *                extents: the AZ neighbours first, which leave most patches
+ *                nothing, before the other fronts are even read;
+ *   per target   of a surviving cluster, one lane each.
+ * The (patch, target) items that remain go to a list, and k_cpa_items
+ * decides their 32 pairs by the FP64 distances, a warp an item: a few
+ * patches hold nearly all of them, and one warp that worked through its own
+ * took ten times as long as the rest of the launch.  The bounds only reject
+ * what those comparisons reject, so they change no result; under
+ * WQ3D_CHECKED the FP64 form takes every target of every patch instead.
+ * A target at the source's latitude and longitude compares its neighbours
+ * by other rules (de_branch); it and its cluster skip the neighbour bounds.
+ *
+ * Bounds.  With mid m_k and half-width h_k of dq_k over the patch's rays,
+ * sum_k w_k m_k + |w_k| h_k is at least every ray's value; a cluster's
+ * weights differ from its centre's by at most D_k, which adds sum_k D_k
+ * (|m_k| + h_k).  Features are formed in FP32 from FP64 coordinate
+ * differences; with A_k the sum of the magnitudes of dq_k's terms over the
+ * patch and W_k the largest |w_k| of all targets, their rounding and the
+ * weights' is below 8 u A_k W_k (u = 2^-24) and that of the 14 products and
+ * sums of a bound below 17 u of 2 sum_k W_k A_k: the guards take 96 u, and
+ * 192 u where a cluster's extents enter.  All add c0 = max(1 m^2, 4e-15 (rho^2 + R^2)) for
+ * the rounding of the reference's FP64 expression on the two points (each
+ * within 5 x 2^-53 (rho^2 + R^2), 0.05 m^2 at earth radius).  A NaN in a ray
+ * or target makes its bounds NaN, which reject nothing.
+ *
+ * Why this shape: per pair the search costs what the bounds let through.
+ * On the sloped workload (1801 x 91 rays, 1024 targets, step 100) the two
+ * fronts alone leave 33 targets per patch, the D/E neighbours 7.9 and the AZ
+ * neighbours 1.7, in 6 % of the patches; a 16 x 8 patch with the fronts
+ * alone, one thread per ray and all targets bounded one by one, left 348.
+ * A launch is then bound by the latency of reading the rays and forming
+ * their ranges: 29 us there and 18 us later on, where nothing survives, with
+ * 4.6 us of k_cpa_items (ncu), for 94 to 103 us before; 264 -> 43 us in the
+ * FP64 form (907 x 53 rays, 667 targets), 1,880 -> 170 us on the
+ * reverberation workload (3601 x 181 rays, 4096 targets). */
 namespace {
-constexpr int F32_TARGETS = CPA_F32_TARGETS;
-struct TgtW {
-    float w[8];
-};
-struct WarpQueue {
-    uint32_t e[64];
-};
+constexpr int CPA_K = 7; /* features */
+enum { CPA_ANEXT, CPA_APREV, CPA_NEXT, CPA_PREV, CPA_DNEXT, CPA_DPREV, CPA_TESTS };
 
-/* finishes queued pairs in FP64: entry = (thread of the ray << 16) | target */
-__device__ __noinline__ void cpa_finish(const QueueDev& q, int64_t s, const FrontPtrs& V, const FrontPtrs& C,
-                           const FrontPtrs& X, const TgtS* tile, int t0, int de0, int az0,
-                           const uint32_t* e, int count, int lane) {
-    if (lane >= count) return;
-    const uint32_t v = e[lane];
-    const int j = (int)(v & 0xffffu);
-    const int th = (int)(v >> 16);
-    WQ_CHECKED_OR(q, j < CPA_F32_TARGETS && th < CPA_THREADS, return);
-    const int de = de0 + th / CPA_PATCH_AZ, az = az0 + th % CPA_PATCH_AZ;
-    const int i = de * q.naz + az;
-    WQ_CHECKED_OR(q, de < q.nde && az < q.naz, return);
-    const TgtS t = tile[j];
-    const double center = d2_at(C, i, t);
-    if (d2_at(X, i, t) <= center) return;
-    if (d2_at(V, i, t) < center) return;
-    double cube[3][3][3];
-    if (!is_closest(q, V, C, X, t, q.de_branch[t0 + j] != 0, de, az, center, cube)) return;
-    cand_push(q, s, (uint32_t)(t0 + j), (uint32_t)i);
-}
-
-/* order-preserving keys of floats, for the warp's unsigned min / max
- * reductions (non-NaN values; -0 orders below +0) */
-__device__ __forceinline__ unsigned f2key(float f) {
-    const unsigned b = __float_as_uint(f);
-    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-__device__ __forceinline__ float key2f(unsigned k) {
-    return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
-}
-
-/* whether every ray of the patch rejects a target on one comparison.  In
- * FP32: each product and the 8-term sums carry at most about 8u of mag
- * (u = 2^-24), the weight sum about 9u of wm, the last three additions
- * about 3u of mag + c0; the 14u, 43u (41u of the per-ray screen plus its
- * own rounding) and 1.0003 factors cover them, so a rejection implies that
- * every ray's FP32 screen rejects the pair. */
-struct PatchGuard {
-    float M[8]; /* max(|lo_k|, |hi_k|) of the patch's feature ranges      */
-    float K;    /* 43u * sum_k W_k M_k (W: the tile's largest weights)     */
-    float Cc;   /* 1.0003 c0                                               */
+struct CpaWarp {
+    float m[CPA_TESTS][8], h[CPA_TESTS][8]; /* feature mid and half-width of each difference */
+    float guard[CPA_TESTS];                 /* sum_k W_k A_k; infinite where not comparable  */
 };
 
-/* the parts of the bound that are the same for every target of the tile */
-__device__ __forceinline__ PatchGuard patch_guard(const float* lo, const float* hi, const float* W, float c0) {
-    PatchGuard p;
-    float wm = 0.0f;
+/* the ray of a lane of a patch */
+struct CpaLane {
+    int de, az, i;
+    bool inside, active;
+};
+
+__device__ __forceinline__ CpaLane cpa_lane(const QueueDev& q, const FrontPtrs& C, const CpaPatch& P, int lane) {
+    CpaLane o;
+    o.de = P.de + (lane >> P.shift);
+    o.az = P.az + (lane & ((1 << P.shift) - 1));
+    o.inside = o.de < q.nde && o.az < q.naz;
+    o.i = o.inside ? o.de * q.naz + o.az : P.de * q.naz + P.az;
+    o.active = o.inside && o.de >= 1 && o.de < q.nde - 1 && o.az >= (q.az_boundary ? 0 : 1) && o.az < q.naz - 1 &&
+               !C.on_edge[o.i];
+    return o;
+}
+
+/* decides the pairs of target j and the rays "rays" (lanes) of a patch by
+ * the FP64 distances; called by a whole warp */
+__device__ __forceinline__ void cpa_item(const QueueDev& q, int64_t s, const FrontPtrs& V, const FrontPtrs& C,
+                                         const FrontPtrs& X, const CpaPatch& P, uint32_t j, unsigned rays, int lane) {
+    const CpaLane L = cpa_lane(q, C, P, lane);
+    const TgtS t{q.tgt[1][j], q.tgt[2][j], q.tgt_sin[j], q.tgt_R2[j], q.tgt_2R[j]};
+    const bool branch = q.de_branch[j] != 0;
+    const double center = d2_at(C, L.i, t), next = d2_at(X, L.i, t), prev = d2_at(V, L.i, t);
+    const int pa = 1 << P.shift;
+    bool hit = L.active && ((rays >> lane) & 1u) && !(next <= center) && !(prev < center);
+    /* the neighbours in the patch, before is_closest loads them all */
+    const double dn = __shfl_down_sync(0xffffffffu, center, pa), dp = __shfl_up_sync(0xffffffffu, center, pa);
+    const unsigned ok = __ballot_sync(0xffffffffu, L.inside && !C.on_edge[L.i]);
+    if (!branch && lane + pa < 32 && ((ok >> (lane + pa)) & 1u) && dn <= center) hit = false;
+    if (!branch && lane >= pa && ((ok >> (lane - pa)) & 1u) && dp < center) hit = false;
+    if (hit && is_closest(q, V, C, X, t, branch, L.de, L.az, center)) cand_push(q, s, j, (uint32_t)L.i);
+}
+
+/* smallest and largest of a warp's values (NaN if any is NaN) */
+__device__ __forceinline__ float warp_min(float v) {
+    float r;
+    asm("redux.sync.min.NaN.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm("redux.sync.max.NaN.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+/* a ray on the curr front, relative to the reference */
+struct CpaRay {
+    double rho, th, ph, rs;
+    float r, x, y;
+};
+
+/* features of point i of front f minus those of the ray; dx, dy: its
+ * theta and phi differences */
+__device__ __forceinline__ void feature_diff(const FrontPtrs& f, int i, const CpaRay& c, float* d, float* dx,
+                                             float* dy) {
+    const double rho = f.cpa[0][i];
+    const double rs = rho * f.cpa[3][i];
+    const float dr = (float)(rho - c.rho), ds = (float)(rs - c.rs);
+    const float tx = (float)(f.cpa[1][i] - c.th), ty = (float)(f.cpa[2][i] - c.ph);
+    const float R = (float)rho, S = (float)rs;
+    d[0] = dr * fmaf(2.0f, c.r, dr);
+    d[1] = dr;
+    d[2] = fmaf(R * tx, fmaf(2.0f, c.x, tx), c.x * c.x * dr);
+    d[3] = fmaf(R, tx, c.x * dr);
+    d[4] = fmaf(S * ty, fmaf(2.0f, c.y, ty), c.y * c.y * ds);
+    d[5] = fmaf(S, ty, c.y * ds);
+    d[6] = ds;
+    *dx = tx;
+    *dy = ty;
+}
+
+/* a point's weights from R, R S and its offsets from the reference */
+__device__ __forceinline__ void target_weights(double R, double RS, double Rr, double X, double Y, float* w) {
+    w[0] = 1.0f;
+    w[1] = (float)(R * X * X - 2.0 * Rr);
+    w[2] = (float)R;
+    w[3] = (float)(-2.0 * R * X);
+    w[4] = (float)RS;
+    w[5] = (float)(-2.0 * RS * Y);
+    w[6] = (float)(RS * Y * Y);
+}
+
+/* the bound's two sums for weights w */
+__device__ __forceinline__ float range_bound(const float* w, const float* m, const float* h) {
+    float a = m[0] + h[0], b = 0.0f;
 #pragma unroll
-    for (int m = 0; m < 8; ++m) {
-        p.M[m] = fmaxf(fabsf(lo[m]), fabsf(hi[m]));
-        wm += W[m] * p.M[m];
+    for (int k = 1; k < CPA_K; ++k) {
+        a = fmaf(w[k], m[k], a);
+        b = fmaf(fabsf(w[k]), h[k], b);
     }
-    const float u = 5.9604645e-8f; /* 2^-24 */
-    p.K = (43.0f * u) * wm;
-    p.Cc = 1.0003f * c0;
-    return p;
-}
-
-/* The sum above with one product per term: rounding is monotone, so
- * max(fl(w lo), fl(w hi)) is fl(w hi) for w >= 0 and fl(w lo) otherwise,
- * and max(|fl(w lo)|, |fl(w hi)|) is fl(|w| max(|lo|, |hi|)); the
- * additions keep their order, so the decisions are those of the full
- * form. */
-__device__ __forceinline__ bool patch_rejects(const TgtW& g, const float* lo, const float* hi,
-                                              const PatchGuard& p) {
-    float ub = 0.0f, mag = 0.0f;
-#pragma unroll
-    for (int m = 0; m < 8; ++m) {
-        const float w = g.w[m];
-        ub += w * (w >= 0.0f ? hi[m] : lo[m]);
-        mag += fabsf(w) * p.M[m];
-    }
-    const float u = 5.9604645e-8f; /* 2^-24 */
-    return ub + (14.0f * u) * mag + p.K + p.Cc < 0.0f;
-}
-}  // namespace
-
-/* FP32 screen value sum_k w_k dq_k as two 4-term chains (any summation
- * order stays within the guard's 8 u bound) */
-__device__ __forceinline__ float screen_dot(const TgtW& g, const float* d) {
-    float a = fmaf(g.w[3], d[3], fmaf(g.w[2], d[2], fmaf(g.w[1], d[1], d[0])));
-    float b = fmaf(g.w[7], d[7], fmaf(g.w[6], d[6], fmaf(g.w[5], d[5], g.w[4] * d[4])));
     return a + b;
 }
 
-/* The patch search; SCREEN decides the per-pair comparisons in FP32 first
- * (FP32C form), otherwise every pair of the patch's surviving targets goes
- * to the FP64 comparisons (FP64 form) */
-template <bool SCREEN>
-__device__ __forceinline__ void cpa_patch(const QueueDev& q, int k) {
-    __shared__ TgtS tile[F32_TARGETS];
-    __shared__ TgtW tw[F32_TARGETS];
-    __shared__ float wmax[CPA_THREADS / 32][8];
-    __shared__ float red[CPA_THREADS / 32][32];
-    __shared__ float bound[32];
-    __shared__ uint16_t surv[F32_TARGETS];
-    __shared__ int nsurv;
-    __shared__ WarpQueue wq[CPA_THREADS / 32];
+/* The ranges of a difference over the lanes "mine" into the warp's slot n,
+ * with its guard; xm, ym, rm: the largest |x|, |y|, |r| of the patch.  Where
+ * a lane of "mine" is not "comparable" the difference rejects nothing. */
+__device__ __forceinline__ void set_range(CpaWarp& S, int n, bool mine, bool comparable, const float* d, float dx,
+                                          float dy, const float* W, float rm, float xm, float ym, int lane) {
+    float mx[CPA_K], hx[CPA_K];
+#pragma unroll
+    for (int k = 0; k < CPA_K; ++k) {
+        const float lo = warp_min(mine ? d[k] : INFINITY), hi = warp_max(mine ? d[k] : -INFINITY);
+        mx[k] = 0.5f * (lo + hi);
+        hx[k] = 1.000001f * fmaxf(hi - mx[k], mx[k] - lo);
+    }
+    const float dxm = warp_max(mine ? fabsf(dx) : 0.0f), dym = warp_max(mine ? fabsf(dy) : 0.0f);
+    const float drm = fabsf(mx[1]) + hx[1], dsm = fabsf(mx[6]) + hx[6];
+    /* A_k: W[2] and W[4] stand for rho and rho sin(theta), which are the
+     * targets' R to within a factor of two */
+    float g = drm * fmaf(2.0f, rm, drm);
+    g = fmaf(W[1], drm, g);
+    g = fmaf(W[2], 2.0f * W[2] * dxm * fmaf(2.0f, xm, dxm) + xm * xm * drm, g);
+    g = fmaf(W[3], 2.0f * W[2] * dxm + xm * drm, g);
+    g = fmaf(W[4], 2.0f * W[2] * dym * fmaf(2.0f, ym, dym) + ym * ym * dsm, g);
+    g = fmaf(W[5], 2.0f * W[2] * dym + ym * dsm, g);
+    g = fmaf(W[6], dsm, g);
+    if (__any_sync(0xffffffffu, mine && !comparable)) g = INFINITY;
+    if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < CPA_K; ++k) {
+            S.m[n][k] = mx[k];
+            S.h[n][k] = hx[k];
+        }
+        S.guard[n] = g;
+    }
+}
+
+/* a cluster's centre weights and the most its targets' differ by */
+struct ClusterW {
+    float w[8], D[8];
+    bool branch;
+};
+
+__device__ __forceinline__ void cluster_weights(const TgtCluster& cl, double rho0, double th0, double ph0,
+                                                ClusterW& o) {
+    const double Xo = cl.T - th0, Yo = cl.P - ph0;
+    target_weights(cl.R, cl.RS, cl.R - rho0, Xo, Yo, o.w);
+    const float ax = fabsf((float)Xo), ay = fabsf((float)Yo);
+    const float Rt = o.w[2] + cl.dR, St = fabsf(o.w[4]) + cl.dRS;
+    o.D[1] = fmaf(2.0f, cl.dR, fmaf(Rt * cl.dT, fmaf(2.0f, ax, cl.dT), ax * ax * cl.dR));
+    o.D[2] = cl.dR;
+    o.D[3] = 2.0f * fmaf(Rt, cl.dT, ax * cl.dR);
+    o.D[4] = cl.dRS;
+    o.D[5] = 2.0f * fmaf(St, cl.dP, ay * cl.dRS);
+    o.D[6] = fmaf(St * cl.dP, fmaf(2.0f, ay, cl.dP), ay * ay * cl.dRS);
+    o.branch = cl.branch != 0;
+}
+
+constexpr float CPA_U = 5.9604645e-8f; /* 2^-24 */
+
+/* whether difference n may be non-negative for some ray and some target of
+ * the cluster */
+__device__ __forceinline__ bool cluster_keeps(const CpaWarp& S, int n, const ClusterW& c, float c0) {
+    float b = 0.0f;
+#pragma unroll
+    for (int k = 1; k < CPA_K; ++k) b = fmaf(c.D[k], fabsf(S.m[n][k]) + S.h[n][k], b);
+    b = fmaf(1.001f, b, range_bound(c.w, S.m[n], S.h[n]));
+    return !(b + fmaf(192.0f * CPA_U, S.guard[n], 1.001f * c0) < 0.0f);
+}
+
+__device__ __forceinline__ bool target_keeps(const CpaWarp& S, int n, const float* w, float c0) {
+    return !(range_bound(w, S.m[n], S.h[n]) + fmaf(96.0f * CPA_U, S.guard[n], 1.001f * c0) < 0.0f);
+}
+}  // namespace
+
+/* four blocks per SM (128 registers) */
+__global__ void __launch_bounds__(32 * CPA_WARPS, 4) k_cpa(__grid_constant__ const QueueDev q, int k) {
+    __shared__ CpaWarp shared[CPA_WARPS];
     const int64_t s = *q.d_base + k + 1;
     const FrontPtrs& V = q.F[ring_slot(s + 1)];
     const FrontPtrs& C = q.F[ring_slot(s + 2)];
     const FrontPtrs& X = q.F[ring_slot(s + 3)];
-    if (q.nde < 3 || q.naz < 3 || q.nt <= 0) return;
-    const int n_pa = (q.naz + CPA_PATCH_AZ - 1) / CPA_PATCH_AZ;
-    const int de0 = (blockIdx.x / n_pa) * CPA_PATCH_DE;
-    const int az0 = (blockIdx.x % n_pa) * CPA_PATCH_AZ;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int de = de0 + threadIdx.x / CPA_PATCH_AZ, az = az0 + threadIdx.x % CPA_PATCH_AZ;
-    bool active = de < q.nde && az < q.naz;
-    const int i = active ? de * q.naz + az : 0;
-    if (active) {
-        const int az_start = q.az_boundary ? 0 : 1;
-        active = !(de < 1 || de >= q.nde - 1 || az < az_start || az >= q.naz - 1) && !C.on_edge[i];
-    }
-    if (!__syncthreads_or(active)) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int wid = blockIdx.x * CPA_WARPS + warp;
+    if (wid >= q.n_patch) return; /* a whole warp: no block barrier follows */
+    CpaWarp& S = shared[warp];
+    const CpaPatch P = q.patches[wid];
+    const int pa = 1 << P.shift;
+    const CpaLane L = cpa_lane(q, C, P, lane);
+    const int az = L.az, i = L.i;
+    const bool inside = L.inside, active = L.active;
+    if (!__any_sync(0xffffffffu, active)) return;
+
     /* local coordinates about the patch's middle ray */
-    const int i_ref = min(de0 + CPA_PATCH_DE / 2, q.nde - 1) * q.naz + min(az0 + CPA_PATCH_AZ / 2, q.naz - 1);
+    const int i_ref = min(P.de + (16 >> P.shift), q.nde - 1) * q.naz + min(P.az + pa / 2, q.naz - 1);
     const double rho0 = C.cpa[0][i_ref], th0 = C.cpa[1][i_ref], ph0 = C.cpa[2][i_ref];
-
-    /* this thread's ray: feature differences next-curr and prev-curr */
-    float dxc[8], dvc[8];
+    CpaRay ray;
+    ray.rho = C.cpa[0][i];
+    ray.th = C.cpa[1][i];
+    ray.ph = C.cpa[2][i];
+    ray.rs = ray.rho * C.cpa[3][i];
+    ray.r = (float)(ray.rho - rho0);
+    ray.x = (float)(ray.th - th0);
+    ray.y = (float)(ray.ph - ph0);
+    const float rm = warp_max(active ? fabsf(ray.r) : 0.0f);
+    const float xm = warp_max(active ? fabsf(ray.x) : 0.0f);
+    const float ym = warp_max(active ? fabsf(ray.y) : 0.0f);
+    /* largest weights of all targets */
+    float W[8];
     {
-        double fq[3][8];
-        const FrontPtrs* fr[3] = {&V, &C, &X};
-#pragma unroll
-        for (int m = 0; m < 3; ++m) {
-            const double rho = fr[m]->cpa[0][i], sn = fr[m]->cpa[3][i];
-            const double r = rho - rho0, x = fr[m]->cpa[1][i] - th0, y = fr[m]->cpa[2][i] - ph0;
-            const double rs = rho * sn;
-            fq[m][0] = r * r;
-            fq[m][1] = r;
-            fq[m][2] = rho * x * x;
-            fq[m][3] = rho * x;
-            fq[m][4] = rho;
-            fq[m][5] = rs * y * y;
-            fq[m][6] = rs * y;
-            fq[m][7] = rs;
-        }
-#pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            dxc[m] = (float)(fq[2][m] - fq[1][m]);
-            dvc[m] = (float)(fq[0][m] - fq[1][m]);
-        }
+        const float Xm = (float)fmax(fabs(q.tgt_box[2] - th0), fabs(q.tgt_box[3] - th0));
+        const float Ym = (float)fmax(fabs(q.tgt_box[4] - ph0), fabs(q.tgt_box[5] - ph0));
+        const float Rm = (float)fmax(fabs(q.tgt_box[0] - rho0), fabs(q.tgt_box[1] - rho0));
+        const float R = 1.0001f * fmaxf((float)q.tgt_box[1], (float)rho0);
+        W[1] = 1.0001f * (R * Xm * Xm + 2.0f * Rm);
+        W[2] = W[4] = R;
+        W[3] = 2.0f * R * Xm;
+        W[5] = 2.0f * R * Ym;
+        W[6] = 1.0001f * R * Ym * Ym;
     }
-    /* feature ranges over the patch's active rays: bound[0..7] / [8..15]
-     * low / high of dxc, [16..23] / [24..31] of dvc */
-#pragma unroll
-    for (int m = 0; m < 8; ++m) {
-        const unsigned l1 = __reduce_min_sync(0xffffffffu, f2key(active ? dxc[m] : INFINITY));
-        const unsigned h1 = __reduce_max_sync(0xffffffffu, f2key(active ? dxc[m] : -INFINITY));
-        const unsigned l2 = __reduce_min_sync(0xffffffffu, f2key(active ? dvc[m] : INFINITY));
-        const unsigned h2 = __reduce_max_sync(0xffffffffu, f2key(active ? dvc[m] : -INFINITY));
-        if (lane == 0) {
-            red[w][m] = key2f(l1);
-            red[w][8 + m] = key2f(h1);
-            red[w][16 + m] = key2f(l2);
-            red[w][24 + m] = key2f(h2);
-        }
+    const float c0 = fmaxf(1.0f, 4.0e-15f * ((float)rho0 * (float)rho0 + W[2] * W[2]));
+
+    /* The AZ neighbours that is_closest compares the ray with: all but the
+     * first and last ray of a fan that does not wrap. */
+    {
+        float d[8], dx, dy;
+        const int an = active ? wrap_az(q, az, 2) : az, ap = active ? wrap_az(q, az, 0) : az;
+        const int row = i - (inside ? az : P.az);
+        feature_diff(C, inside ? row + an : i, ray, d, &dx, &dy);
+        set_range(S, CPA_ANEXT, active, an != q.naz - 1 && (an != 0 || q.az_boundary), d, dx, dy, W, rm, xm, ym, lane);
+        feature_diff(C, inside ? row + ap : i, ray, d, &dx, &dy);
+        set_range(S, CPA_APREV, active, ap != q.naz - 1 && (ap != 0 || q.az_boundary), d, dx, dy, W, rm, xm, ym, lane);
     }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        const bool low = (threadIdx.x & 8) == 0;
-        float v = red[0][threadIdx.x];
-        for (int j = 1; j < CPA_THREADS / 32; ++j) v = low ? fminf(v, red[j][threadIdx.x]) : fmaxf(v, red[j][threadIdx.x]);
-        bound[threadIdx.x] = v;
+    __syncwarp();
+    /* this warp's share of the clusters; nothing more to do for most warps */
+    const int ncl = (q.nt + 31) >> 5;
+    const int per = (ncl + P.parts - 1) / P.parts;
+    const int c_begin = P.part * per, c_end = min(ncl, c_begin + per);
+    {
+        bool keep = false;
+        for (int c = c_begin + lane; c < c_end && !keep; c += 32) {
+            ClusterW cw;
+            cluster_weights(q.clusters[c], rho0, th0, ph0, cw);
+            keep = cw.branch || (cluster_keeps(S, CPA_ANEXT, cw, c0) && cluster_keeps(S, CPA_APREV, cw, c0));
+        }
+#if WQ3D_CHECKED
+        keep = keep || q.precision == WQ3D_FP64;
+#endif
+        if (!__any_sync(0xffffffffu, keep)) return;
     }
 
-    uint32_t* myq = wq[w].e;
+    /* the ray on the next and prev fronts, and its D/E neighbours (those on
+     * an edge are not compared) */
+    float dx[8], dv[8], dn[8], dp[8], tx[4], ty[4];
+    feature_diff(X, i, ray, dx, &tx[0], &ty[0]);
+    feature_diff(V, i, ray, dv, &tx[1], &ty[1]);
+    const int in = active ? i + q.naz : i, ip = active ? i - q.naz : i;
+    feature_diff(C, in, ray, dn, &tx[2], &ty[2]);
+    feature_diff(C, ip, ray, dp, &tx[3], &ty[3]);
+    const bool edge_n = C.on_edge[in] != 0, edge_p = C.on_edge[ip] != 0;
+
+    /* appends the items of this patch's rays "rays" and the lanes' targets
+     * to the step's list; one that finds no room is decided here */
+    const int list = (int)(s & 1);
     const unsigned lt = (1u << lane) - 1u;
-    const float u = 5.9604645e-8f;
-    /* this block's tile of targets (grid.y splits a patch's targets) */
+    auto append = [&](bool want, uint32_t t, unsigned rays) {
+        unsigned mask = __ballot_sync(0xffffffffu, want);
+        if (!mask) return;
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(q.n_item + list, (uint32_t)__popc(mask));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        const uint32_t slot = base + (uint32_t)__popc(mask & lt);
+        const bool fits = slot < q.cap_item;
+        if (want && fits) q.items[slot] = make_uint4((uint32_t)wid, t, rays, 0u);
+        mask = __ballot_sync(0xffffffffu, want && !fits);
+        while (mask) {
+            const uint32_t tl = __shfl_sync(0xffffffffu, t, __ffs(mask) - 1);
+            mask &= mask - 1;
+            cpa_item(q, s, V, C, X, P, tl, rays, lane);
+        }
+    };
+#if WQ3D_CHECKED
+    if (q.precision == WQ3D_FP64) {
+        for (int j0 = c_begin * 32; j0 < min(q.nt, c_end * 32); j0 += 32) {
+            const int j = j0 + lane;
+            append(j < q.nt, j < q.nt ? q.cpa_index[j] : 0u, 0xffffffffu);
+        }
+        return;
+    }
+#endif
+
+    /* Rays that have just met a boundary move unlike their neighbours, and
+     * one range over both would let most targets through: where the radial
+     * parts of a patch's steps differ by more than 0.3 of its longest step,
+     * the rays on either side of the middle are searched on their own. */
+    int key = 0;
     {
-        const int t0 = blockIdx.y * F32_TARGETS;
-        if (t0 >= q.nt) return;
-        const int nt_tile = min(F32_TARGETS, q.nt - t0);
-        float W[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int j = threadIdx.x; j < nt_tile; j += blockDim.x) {
-            const int t = t0 + j;
-            const double R = q.tgt[0][t], T = q.tgt[1][t], P = q.tgt[2][t], S = q.tgt_sin[t];
-            tile[j] = TgtS{T, P, S, q.tgt_R2[t], q.tgt_2R[t]};
-            const double Rr = R - rho0, Xo = T - th0, Yo = P - ph0, RS = R * S;
-            TgtW g;
-            g.w[0] = 1.0f;
-            g.w[1] = (float)(-2.0 * Rr);
-            g.w[2] = (float)R;
-            g.w[3] = (float)(-2.0 * R * Xo);
-            g.w[4] = (float)(R * Xo * Xo);
-            g.w[5] = (float)RS;
-            g.w[6] = (float)(-2.0 * RS * Yo);
-            g.w[7] = (float)(RS * Yo * Yo);
-            tw[j] = g;
-#pragma unroll
-            for (int m = 0; m < 8; ++m) W[m] = fmaxf(W[m], fabsf(g.w[m]));
-        }
-        /* W >= 0: its bit patterns order as unsigned integers */
-#pragma unroll
-        for (int m = 0; m < 8; ++m)
-            W[m] = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(W[m])));
-        if (lane == 0)
-            for (int m = 0; m < 8; ++m) wmax[w][m] = W[m];
-        if (threadIdx.x == 0) nsurv = 0;
-        __syncthreads();
-#pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            float v = 0.0f;
-            for (int j = 0; j < CPA_THREADS / 32; ++j) v = fmaxf(v, wmax[j][m]);
-            W[m] = v * 1.0001f;
-        }
-        /* the guards of this tile, per ray and for the patch bound */
-        const float r0 = (float)rho0;
-        const float c0 = fmaxf(1.0f, 4.0e-15f * (r0 * r0 + W[2] * W[2]));
-        float gxc = 0.0f, gvc = 0.0f;
-#pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            gxc = fmaf(W[m], fabsf(dxc[m]), gxc);
-            gvc = fmaf(W[m], fabsf(dvc[m]), gvc);
-        }
-        gxc = fmaf(32.0f * u, gxc, c0);
-        gvc = fmaf(32.0f * u, gvc, c0);
-        /* targets that some ray of the patch may keep */
-        const PatchGuard px = patch_guard(&bound[0], &bound[8], W, c0);
-        const PatchGuard pv = patch_guard(&bound[16], &bound[24], W, c0);
-        for (int j = threadIdx.x; j < nt_tile; j += blockDim.x) {
-            const TgtW g = tw[j];
-            if (patch_rejects(g, &bound[0], &bound[8], px)) continue;
-            if (patch_rejects(g, &bound[16], &bound[24], pv)) continue;
-            surv[atomicAdd(&nsurv, 1)] = (uint16_t)j;
-        }
-        __syncthreads();
-        const int ns = nsurv;
-        int qn = 0;
-        /* appends this lane's pair if "want"; finishes 32 at a time */
-        auto push = [&](bool want, int j) {
-            const unsigned mask = __ballot_sync(0xffffffffu, want);
-            if (mask) {
-                if (want) myq[qn + __popc(mask & lt)] = ((uint32_t)threadIdx.x << 16) | (uint32_t)j;
-                qn += __popc(mask);
-                __syncwarp();
-                if (qn >= 32) {
-                    cpa_finish(q, s, V, C, X, tile, t0, de0, az0, myq, 32, lane);
-                    __syncwarp();
-                    if (lane < qn - 32) myq[lane] = myq[32 + lane];
-                    __syncwarp();
-                    qn -= 32;
+        const float len = warp_max(active ? fmaxf(fabsf(dx[1]), fmaxf(fabsf(dx[3]), fabsf(dx[5]))) : 0.0f);
+        const float lx = warp_min(active ? dx[1] : INFINITY), hx = warp_max(active ? dx[1] : -INFINITY);
+        const float lv = warp_min(active ? dv[1] : INFINITY), hv = warp_max(active ? dv[1] : -INFINITY);
+        if (hx - lx > 0.3f * len && dx[1] > 0.5f * (lx + hx)) key |= 1;
+        if (hv - lv > 0.3f * len && dv[1] > 0.5f * (lv + hv)) key |= 2;
+    }
+
+    unsigned left = __ballot_sync(0xffffffffu, active);
+    while (left) {
+        const int lead = __shfl_sync(0xffffffffu, key, __ffs(left) - 1); /* every lane takes part */
+        const bool mine = active && key == lead;
+        const unsigned group = __ballot_sync(0xffffffffu, mine);
+        left &= ~group;
+        __syncwarp();
+        set_range(S, CPA_NEXT, mine, true, dx, tx[0], ty[0], W, rm, xm, ym, lane);
+        set_range(S, CPA_PREV, mine, true, dv, tx[1], ty[1], W, rm, xm, ym, lane);
+        set_range(S, CPA_DNEXT, mine, !edge_n, dn, tx[2], ty[2], W, rm, xm, ym, lane);
+        set_range(S, CPA_DPREV, mine, !edge_p, dp, tx[3], ty[3], W, rm, xm, ym, lane);
+        __syncwarp();
+        for (int cb = c_begin; cb < c_end; cb += 32) {
+            bool keep = false;
+            if (cb + lane < c_end) {
+                ClusterW cw;
+                cluster_weights(q.clusters[cb + lane], rho0, th0, ph0, cw);
+                keep = cluster_keeps(S, CPA_NEXT, cw, c0) && cluster_keeps(S, CPA_PREV, cw, c0);
+                if (keep && !cw.branch)
+                    keep = cluster_keeps(S, CPA_ANEXT, cw, c0) && cluster_keeps(S, CPA_APREV, cw, c0) &&
+                           cluster_keeps(S, CPA_DNEXT, cw, c0) && cluster_keeps(S, CPA_DPREV, cw, c0);
+            }
+            unsigned cmask = __ballot_sync(0xffffffffu, keep);
+            while (cmask) {
+                const int j = ((cb + __ffs(cmask) - 1) << 5) + lane;
+                cmask &= cmask - 1;
+                bool want = false;
+                uint32_t t = 0;
+                if (j < q.nt) {
+                    const double2 a = __ldg(reinterpret_cast<const double2*>(q.cpa_tgt) + 2 * (size_t)j);
+                    const double2 b = __ldg(reinterpret_cast<const double2*>(q.cpa_tgt) + 2 * (size_t)j + 1);
+                    t = __ldg(q.cpa_index + j);
+                    float w[8];
+                    target_weights(a.x, a.x * b.y, a.x - rho0, a.y - th0, b.x - ph0, w);
+                    want = target_keeps(S, CPA_NEXT, w, c0) && target_keeps(S, CPA_PREV, w, c0);
+                    if (want && q.de_branch[t] == 0)
+                        want = target_keeps(S, CPA_ANEXT, w, c0) && target_keeps(S, CPA_APREV, w, c0) &&
+                               target_keeps(S, CPA_DNEXT, w, c0) && target_keeps(S, CPA_DPREV, w, c0);
                 }
+                append(want, t, group);
             }
-        };
-        int sidx = 0;
-        for (; sidx + 1 < ns; sidx += 2) {
-            const int j0 = surv[sidx], j1 = surv[sidx + 1];
-            const TgtW g0 = tw[j0], g1 = tw[j1];
-            bool w0 = active, w1 = active;
-            if (SCREEN) {
-                const float a0 = screen_dot(g0, dxc), a1 = screen_dot(g1, dxc);
-                w0 = w0 && !(a0 < -gxc);
-                w1 = w1 && !(a1 < -gxc);
-                if (w0 || w1) {
-                    const float b0 = screen_dot(g0, dvc), b1 = screen_dot(g1, dvc);
-                    w0 = w0 && !(b0 < -gvc);
-                    w1 = w1 && !(b1 < -gvc);
-                }
-            }
-            push(w0, j0);
-            push(w1, j1);
         }
-        if (sidx < ns) {
-            const int j = surv[sidx];
-            const TgtW g = tw[j];
-            bool want = active;
-            if (SCREEN) {
-                want = want && !(screen_dot(g, dxc) < -gxc);
-                if (want) want = !(screen_dot(g, dvc) < -gvc);
-            }
-            push(want, j);
-        }
-        if (qn > 0) cpa_finish(q, s, V, C, X, tile, t0, de0, az0, myq, qn, lane);
     }
 }
 
-/* four resident blocks (128 registers): the reflection chain that runs
- * beside the search keeps issue slots */
-__global__ void __launch_bounds__(CPA_THREADS, 3) k_cpa_f32(__grid_constant__ const QueueDev q, int k) {
-    cpa_patch<true>(q, k);
-}
-
-__global__ void __launch_bounds__(CPA_THREADS, 3) k_cpa(__grid_constant__ const QueueDev q, int k) {
-    cpa_patch<false>(q, k);
+/* the items that k_cpa left, a warp each */
+__global__ void __launch_bounds__(128) k_cpa_items(__grid_constant__ const QueueDev q, int k) {
+    const int64_t s = *q.d_base + k + 1;
+    const FrontPtrs& V = q.F[ring_slot(s + 1)];
+    const FrontPtrs& C = q.F[ring_slot(s + 2)];
+    const FrontPtrs& X = q.F[ring_slot(s + 3)];
+    const int lane = threadIdx.x & 31;
+    const uint32_t n = min(q.n_item[s & 1], q.cap_item);
+    for (uint32_t e = blockIdx.x * 4 + (threadIdx.x >> 5); e < n; e += gridDim.x * 4) {
+        const uint4 it = q.items[e];
+        WQ_CHECKED_OR(q, it.x < (uint32_t)q.n_patch && it.y < (uint32_t)q.nt, continue);
+        cpa_item(q, s, V, C, X, q.patches[it.x], it.y, it.z, lane);
+    }
+    /* the next step's count (its k_cpa follows this launch on the stream;
+     * the step before last used it) */
+    if (blockIdx.x == 0 && threadIdx.x == 0) q.n_item[(s + 1) & 1] = 0;
 }
 
 /* ------------------------------------------------------------------ */
