@@ -1778,8 +1778,8 @@ int wq3d_queue_create(const wq3d_ocean* ocean, const wq3d_queue_desc* d, wq3d_qu
          * all five, and the first step writes the fifth before it is read
          * (zeroing the whole ring cost the 512-queue batch seconds of its
          * build) */
-        if (cudaMemset(base + RING * per_front, 0, 2 * bbytes) != cudaSuccess)
-            return cleanup(fail(WQ3D_ERR_CUDA, "cudaMemset failed"));
+        if (cudaMemsetAsync(base + RING * per_front, 0, 2 * bbytes, q->stream) != cudaSuccess)
+            return cleanup(fail(WQ3D_ERR_CUDA, "cudaMemsetAsync failed"));
         char* p = base;
         auto dtake = [&](size_t count) {
             double* r = reinterpret_cast<double*>(p);
@@ -1857,8 +1857,8 @@ int wq3d_queue_create(const wq3d_ocean* ocean, const wq3d_queue_desc* d, wq3d_qu
     }
     /* no ray reflected in the step before the first */
     for (int p = 0; p < SHADOW_SETS; ++p)
-        if (cudaMemset(h.commit_flag[p], 0, n) != cudaSuccess)
-            return cleanup(fail(WQ3D_ERR_CUDA, "cudaMemset failed"));
+        if (cudaMemsetAsync(h.commit_flag[p], 0, n, q->stream) != cudaSuccess)
+            return cleanup(fail(WQ3D_ERR_CUDA, "cudaMemsetAsync failed"));
     h.d_base = q->d_base;
     h.d_times = q->d_times;
     h.want_refl = 0;
@@ -1874,8 +1874,13 @@ int wq3d_queue_create(const wq3d_ocean* ocean, const wq3d_queue_desc* d, wq3d_qu
             q->h_times[s] = reinterpret_cast<double*>(b + 128);
         }
     }
-    if (cudaMemset(q->d_counts, 0, 24 * sizeof(uint32_t)) != cudaSuccess)
-        return cleanup(fail(WQ3D_ERR_CUDA, "cudaMemset failed"));
+    if (cudaMemsetAsync(q->d_counts, 0, 24 * sizeof(uint32_t), q->stream) != cudaSuccess)
+        return cleanup(fail(WQ3D_ERR_CUDA, "cudaMemsetAsync failed"));
+    /* The queue's streams do not wait for the default stream, on which the
+     * uploads above were made: the start-up must follow the zeroed counters
+     * (cleared on its own stream) and the last of those copies. */
+    if (cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess)
+        return cleanup(fail(WQ3D_ERR_CUDA, "upload failed"));
 
     /* wave_queue ctor: init_wave, update, init_wavefronts */
     q->gridded = ocean->dev.prof.kind == WQ3D_PROFILE_GRID || ocean->dev.surf.kind == WQ3D_BOUNDARY_GRID ||
@@ -2207,7 +2212,7 @@ int wq3d_queue_enable_sensitivity(wq3d_queue* q) {
     if (!rc) rc = q->alloc(&q->h.rec_sens, (size_t)q->h.cap_rec * 3);
     if (!rc && q->have_set1) rc = q->alloc(&q->set1.rec_sens, (size_t)q->h.cap_rec * 3);
     if (rc) return rc;
-    WQ_CK(cudaMemset(dA, 0, RING * 3 * n * sizeof(double)));
+    WQ_CK(cudaMemsetAsync(dA, 0, RING * 3 * n * sizeof(double), q->stream));
     for (int f = 0; f < RING; ++f) q->h.F[f].dA = dA + (size_t)f * 3 * n;
     q->h.sens = 1;
     q->drop_graph();
@@ -2247,7 +2252,7 @@ int wq3d_queue_enable_adjoint(wq3d_queue* q, int checkpoint_interval, size_t max
     int rc = q->alloc(&ck, (size_t)nckpt * ADJ_S * n);
     if (!rc) rc = q->alloc(&rec, cap);
     if (rc) return rc;
-    WQ_CK(cudaMemset(q->d_counts + 11, 0, 2 * sizeof(uint32_t)));
+    WQ_CK(cudaMemsetAsync(q->d_counts + 11, 0, 2 * sizeof(uint32_t), q->stream));
     q->h.adj = 1;
     q->h.adj_K = checkpoint_interval;
     q->h.adj_nckpt = nckpt;
