@@ -1451,6 +1451,27 @@ __global__ void k_adj_touch(AdjSweep a, __grid_constant__ const QueueDev q) {
     }
 }
 
+/* the ray's states as k_adj_recompute's reflection chain leaves them, and
+ * the chain's code; at most eight bounces */
+struct AdjOut {
+    RayS v, c, x;
+    uint32_t code;
+    __device__ void put(int which, const RayS& y) {
+        if (which == 0) v = y;
+        else if (which == 1) c = y;
+        else x = y;
+    }
+    __device__ bool losses() const { return false; }
+    __device__ void add(const Loss&) {}
+    __device__ void tangents(const double*) {}
+    __device__ void bounced(bool bottom) { code = chain_add(code, bottom); }
+    __device__ bool stop(int) {
+        if (((code >> 16) & 0xf) < 8) return false;
+        code |= 0x80000000u;
+        return true;
+    }
+};
+
 /* S_m0 .. S_m1-1 of each ray seeded at or after m0, and each step's
  * reflection chain, with the engine's own step functions */
 __global__ void __launch_bounds__(128) k_adj_recompute(AdjSweep a, __grid_constant__ const QueueDev q) {
@@ -1459,7 +1480,7 @@ __global__ void __launch_bounds__(128) k_adj_recompute(AdjSweep a, __grid_consta
     if ((int64_t)a.last[i] - 1 < a.m0) return;
     const int n = q.n;
     const double* ck = q.adj_ckpt + (size_t)a.ckpt * ADJ_S * n;
-    RayLocal L;
+    AdjOut L;
     RayS* Y[3] = {&L.v, &L.c, &L.x};
     for (int r = 0; r < 3; ++r) {
         for (int c = 0; c < 3; ++c) {
@@ -1469,12 +1490,6 @@ __global__ void __launch_bounds__(128) k_adj_recompute(AdjSweep a, __grid_consta
         Y[r]->dist = 0.0;
         update1(q, *Y[r]);
     }
-    for (int f = 0; f < q.nf; ++f) {
-        L.att[f] = 0.0;
-        L.ph[f] = 0.0;
-    }
-    L.surface = L.bottom = L.caustic = 0;
-    double dl[3] = {0.0, 0.0, 0.0};
     for (int64_t m = a.m0; m < a.m1; ++m) {
         const int64_t j = m - a.m0;
         double* S = a.seg + (size_t)j * ADJ_S * n;
@@ -1483,42 +1498,13 @@ __global__ void __launch_bounds__(128) k_adj_recompute(AdjSweep a, __grid_consta
                 S[(size_t)(r * 6 + c) * n + i] = Y[r]->pos[c];
                 S[(size_t)(r * 6 + 3 + c) * n + i] = Y[r]->nd[c];
             }
-        /* k_reflect's chain (wave_queue.cc:197-256) */
-        uint32_t code = 0;
+        L.code = 0;
         if (reflect_decision(q, L.x.pos, L.c.nd)) {
-            int seq = 0;
-            int next_try = -1;
-            if (L.x.pos[0] - q.R > 0.0 && surface_local(q, q.F[0], L, i, m + 1, 0.0, seq)) {
-                code = chain_add(code, false);
-                next_try = 0;
-            } else {
-                const double depth = boundary_height(q.oc.bot, L.x.pos[1], L.x.pos[2]) - L.x.pos[0];
-                if (depth > 0.0) {
-                    bottom_local(q, q.F[0], L, i, depth, m + 1, 0.0, seq, dl);
-                    code = chain_add(code, true);
-                    next_try = 1;
-                }
-            }
-            if (next_try >= 0) {
-                for (int it = 0; it < MAX_BOUNCE; ++it) {
-                    if (((code >> 16) & 0xf) >= 8) {
-                        code |= 0x80000000u;
-                        break;
-                    }
-                    if (next_try == 0) {
-                        const double depth = boundary_height(q.oc.bot, L.x.pos[1], L.x.pos[2]) - L.x.pos[0];
-                        if (!(depth > 0.0)) break;
-                        bottom_local(q, q.F[0], L, i, depth, m + 1, 0.0, seq, dl);
-                        code = chain_add(code, true);
-                        next_try = 1;
-                    } else {
-                        if (!(L.x.pos[0] - q.R > 0.0 && surface_local(q, q.F[0], L, i, m + 1, 0.0, seq))) break;
-                        code = chain_add(code, false);
-                        next_try = 0;
-                    }
-                }
-            }
+            int surface = 0, bottom = 0;
+            RayC rv = rayc_of(L.v), rc = rayc_of(L.c), rx = rayc_of(L.x);
+            bounce_chain(q, q.F[0], i, m + 1, 0.0, rv, rc, rx, surface, bottom, L);
         }
+        const uint32_t code = L.code;
         if (code & 0x80000000u) atomicOr(a.err, ADJ_ERR_CHAIN);
         a.chain[(size_t)j * n + i] = code;
         if (m + 1 < a.m1) {

@@ -1635,6 +1635,9 @@ int wq3d_queue_create(const wq3d_ocean* ocean, const wq3d_queue_desc* d, wq3d_qu
     h.nt1 = nt ? (int)d->num_targets1 : 0;
     h.nt2 = nt ? (int)d->num_targets2 : 1;
     h.dt = d->time_step;
+    h.r_2dt = 1.0 / (2.0 * h.dt);
+    h.r_dt2 = 1.0 / (h.dt * h.dt);
+    h.dt_ok = h.dt > 1e-30 && h.dt < 1e30 && divisor_ok(2.0 * h.dt) && divisor_ok(h.dt * h.dt);
     h.R = d->earth_radius;
     h.spreading = d->spreading;
     h.precision = d->precision;

@@ -155,6 +155,8 @@ struct QueueDev {
     int spreading;
     int precision;
     double dt;
+    double r_2dt, r_dt2;     /* 1 / (2 dt) and 1 / dt^2                 */
+    int dt_ok;               /* whether quot() may divide by 2 dt, dt^2 */
     double R;
     /* fans and frequencies */
     const double* freq;

@@ -154,24 +154,8 @@ __device__ __forceinline__ void ab3(double h, const RayS& y0, const RayS& y1,
     }
 }
 
-#if !WQ3D_STEP_KERNELS_ONLY
-/* one ray's state (k_volume) */
-__device__ __forceinline__ void load_ray(const FrontPtrs& f, int r, RayS& y) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        y.pos[k] = f.pos[k][r];
-        y.pg[k] = f.pg[k][r];
-        y.nd[k] = f.nd[k][r];
-        y.ng[k] = f.ng[k][r];
-        y.sg[k] = f.sg[k][r];
-    }
-    y.c = f.c[r];
-    y.dist = f.dist[r];
-}
-#endif
-
-/* load_ray through the read-only data cache, for kernels that never write
- * the arrays they read this way: the loads may then all be in flight at
+/* one ray's state through the read-only data cache, for kernels that never
+ * write the arrays they read this way: the loads may then all be in flight at
  * once instead of waiting behind stores to the caller's copy */
 __device__ __forceinline__ void load_ray_ro(const FrontPtrs& f, int r, RayS& y) {
     double v[17];
@@ -272,49 +256,70 @@ __device__ void collision_location(const QueueDev& q, const FrontPtrs& V,
 }
 #endif
 
-/* One reflecting ray's prev/curr/next state and next-front losses, held
- * privately while k_reflect works on it.  The results go to a shadow slot
- * that k_advance commits, so k_cpa / k_eigenray of the previous step can
- * read the fronts at the same time.  (The reference also rewrites the
- * ray's "past" entry, reflection_model.cc:320, but the AB3 step of the
- * same wave_queue::step overwrites that entry before anything reads it.) */
-struct RayLocal {
-    RayS v, c, x;
-    double att[MAX_FREQ];
-    double ph[MAX_FREQ];
-    double phf[MAX_FREQ];  /* the phases had the caustic hand-off shifted them first */
-    int surface, bottom, caustic;
+/* What a reflection reads of a ray on one front.  The reflection chain
+ * keeps these of the prev, curr and next fronts in registers; the whole
+ * states go to the ray's shadow slot as they are made, from which k_advance
+ * and k_commit take them, so k_cpa / k_eigenray of the previous step can
+ * read the fronts at the same time.  (The reference also rewrites the ray's
+ * "past" entry, reflection_model.cc:320, but the AB3 step of the same
+ * wave_queue::step overwrites that entry before anything reads it.) */
+struct RayC {
+    double pos[3], nd[3], c;
 };
 
-/* collision_location (wave_queue.cc:982-1057) from one ray's prev, curr
- * and next states */
-__device__ void collision_rays(const QueueDev& q, const RayS& V, const RayS& Cr, const RayS& X,
-                               double tw, double* pos, double* nd, double* speed) {
+/* a front's or a slot's state (17 doubles), without the slopes */
+__device__ __forceinline__ void load_rayc(const FrontPtrs& f, int r, RayC& y) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        y.pos[k] = __ldg(f.pos[k] + r);
+        y.nd[k] = __ldg(f.nd[k] + r);
+    }
+    y.c = __ldg(f.c + r);
+}
+__device__ __forceinline__ void rayc_from(const double* src, RayC& y) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        y.pos[k] = src[k];
+        y.nd[k] = src[6 + k];
+    }
+    y.c = src[12];
+}
+__device__ __forceinline__ RayC rayc_of(const RayS& y) {
+    RayC o;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        o.pos[k] = y.pos[k];
+        o.nd[k] = y.nd[k];
+    }
+    o.c = y.c;
+    return o;
+}
+
+/* a / r.b, by quot() when the time step's powers are in its range */
+__device__ __forceinline__ double div_dt(const QueueDev& q, double a, Recip r) { return q.dt_ok ? quot(a, r) : a / r.b; }
+
+/* wave_queue::collision_location (wave_queue.cc:982-1057) from one ray's
+ * prev, curr and next states */
+__device__ __forceinline__ void collision_rays(const QueueDev& q, const RayC& V, const RayC& Cr, const RayC& X,
+                                               double tw, double* pos, double* nd, double* speed) {
     const double dt = q.dt;
-    const double time1 = 2.0 * dt;
-    const double time2 = dt * dt;
+    const Recip time1{2.0 * dt, q.r_2dt}, time2{dt * dt, q.r_dt2};
     const double dtime2 = tw * tw;
-    const double drho = (X.c - V.c) / time1;
-    const double d2rho = (X.c + V.c - 2.0 * Cr.c) / time2;
+    const double drho = div_dt(q, X.c - V.c, time1);
+    const double d2rho = div_dt(q, X.c + V.c - 2.0 * Cr.c, time2);
     *speed = Cr.c + drho * tw + 0.5 * d2rho * dtime2;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const double v1 = (X.pos[k] - V.pos[k]) / time1;
-        const double v2 = (X.pos[k] + V.pos[k] - 2.0 * Cr.pos[k]) / time2;
+        const double v1 = div_dt(q, X.pos[k] - V.pos[k], time1);
+        const double v2 = div_dt(q, X.pos[k] + V.pos[k] - 2.0 * Cr.pos[k], time2);
         pos[k] = Cr.pos[k] + v1 * tw + 0.5 * v2 * dtime2;
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const double v1 = (X.nd[k] - V.nd[k]) / time1;
-        const double v2 = (X.nd[k] + V.nd[k] - 2.0 * Cr.nd[k]) / time2;
+        const double v1 = div_dt(q, X.nd[k] - V.nd[k], time1);
+        const double v2 = div_dt(q, X.nd[k] + V.nd[k] - 2.0 * Cr.nd[k], time2);
         nd[k] = Cr.nd[k] + v1 * tw + 0.5 * v2 * dtime2;
     }
-}
-
-/* collision_location on the private state */
-__device__ __forceinline__ void collision_local(const QueueDev& q, const RayLocal& L, double tw,
-                                                double* pos, double* nd, double* speed) {
-    collision_rays(q, L.v, L.c, L.x, tw, pos, nd, speed);
 }
 
 /* seq_vector::increment: the index clamps to the last element, and -1
@@ -394,7 +399,7 @@ __device__ __noinline__ void build_eigenverb(const QueueDev& q, const FrontPtrs&
  * ray's prev / curr / next states V, Cr, X.  The collision time is
  * measured to the ocean surface, not to the layer, as in the reference. */
 __device__ __noinline__ void volume_scatter(const QueueDev& q, const FrontPtrs& C, int i, int64_t step,
-                               double t_old, const RayS& V, const RayS& Cr, const RayS& X,
+                               double t_old, const RayC& V, const RayC& Cr, const RayC& X,
                                int surface, int bottom, int& seq) {
     if (bottom > q.max_bottom || surface > q.max_surface || C.caustic[i] > q.max_caustic ||
         C.upper[i] > q.max_upper || C.lower[i] > q.max_lower)
@@ -415,58 +420,147 @@ __device__ __noinline__ void volume_scatter(const QueueDev& q, const FrontPtrs& 
     }
 }
 
-/* The updates of the re-initialisation, out of line: inlined, they keep
- * the temporary rays in registers, but the larger code made k_reflect
- * wait on instruction fetch (90.6 instead of 58.4 us per launch on the
- * sloped workload, ncu: "no instruction" stalls 2.9 -> 10.1 per issue). */
-__device__ __noinline__ void reinit_update(const QueueDev& q, RayS& y) {
-    if (q.precision == WQ3D_FP32)
-        update1_f32(q, y);
-    else
-        update1(q, y);
+/* update1_f32 out of line: the FP32 form's path through the one update that
+ * the re-initialisation inlines */
+__device__ __noinline__ void reinit_update_f32(const QueueDev& q, RayS& y) { update1_f32(q, y); }
+
+/* wave_front::update of the re-initialisation; *st: sin(theta) */
+__device__ __forceinline__ void reinit_update(const QueueDev& q, RayS& y, double* st) {
+    if (q.precision == WQ3D_FP32) {
+        RayS t = y;
+        reinit_update_f32(q, t);
+        y = t;
+        *st = sin(y.pos[1]);
+    } else {
+        profile_at(q, y.pos, &y.c, y.sg);
+        ray_derivs<!WQ3D_WITH_GRID>(y.c, y.sg[0], y.sg[1], y.sg[2], y.pos, y.nd, y.pg, y.ng, st);
+    }
 }
 
-/* reflection_model::reflection_reinit on the private state */
-__device__ __noinline__ void reinit_local(const QueueDev& q, RayLocal& L, double tw, const double* pos,
-                             const double* nd) {
-    RayS past1, prev1, curr1, next1, temp;
+/* reflection_model::reflection_reinit: from the collision point back to
+ * the times of the curr, prev and past fronts by RK3, and forward to the
+ * next by AB3.  v, c, x take the new prev, curr and next; "out" takes the
+ * whole states (out.put(0 prev / 1 curr / 2 next, state)).
+ *
+ * Ten updates follow one another and bound the chain of a reflecting ray,
+ * and so the step.  They run as ten rounds of one loop with one inlined
+ * copy of the update: the states stay in registers, and the code is small
+ * enough to stay in the instruction cache.  Per step in k_reflect, against
+ * out-of-line updates on states in local memory: 38 for 60 us on the sloped
+ * workload, 60 for 108 us on 901 x 45 rays over a gridded ocean, 49 for 88 us
+ * on STD14.  (Ten inlined copies of the update waited on instruction
+ * fetch.) */
+template <class Out>
+__device__ __forceinline__ void reinit_ray(const QueueDev& q, RayC& v, RayC& c, RayC& x, double tw, const double* pos,
+                                           const double* nd, Out& out) {
+    struct Slope {
+        double p[3], n[3];
+    };
+    RayS y;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        temp.pos[k] = pos[k];
-        temp.nd[k] = nd[k];
+        y.pos[k] = pos[k];
+        y.nd[k] = nd[k];
     }
-    next1.dist = 0.0;
-    past1.dist = 0.0;
-    prev1.dist = 0.0;
-    curr1.dist = 0.0;
-    temp.dist = 0.0;
-    reinit_update(q, temp);
-    rk1(-tw, temp, next1);
-    reinit_update(q, next1);
-    rk2(-tw, temp, next1, past1);
-    reinit_update(q, past1);
-    rk3(-tw, temp, next1, past1, curr1);
-    reinit_update(q, curr1);
-
-    const double h = q.dt;
-    rk1(-h, curr1, next1);
-    reinit_update(q, next1);
-    rk2(-h, curr1, next1, past1);
-    reinit_update(q, past1);
-    rk3(-h, curr1, next1, past1, prev1);
-    reinit_update(q, prev1);
-
-    rk1(-h, prev1, next1);
-    reinit_update(q, next1);
-    rk2(-h, prev1, next1, temp);
-    rk3(-h, prev1, next1, temp, past1);
-    reinit_update(q, past1);
-
-    ab3(h, past1, prev1, curr1, next1);
-    reinit_update(q, next1);
-    L.c = curr1;
-    L.v = prev1;
-    L.x = next1;
+    y.dist = 0.0;
+    double bp[3], bn[3];           /* the state an RK3 run starts from */
+    Slope b0, k1, k2, t0, sc, sv;  /* its slopes, the run's, the collision point's, curr's, prev's */
+    double h = -tw, st, st_c = 0.0;
+    /* rounds: 0 the collision point; 1 2 3 RK3 to curr; 4 5 6 to prev; 7 8
+     * to past (whose second slope is the collision point's: the reference
+     * does not update there); 9 AB3 to next */
+#pragma unroll 1
+    for (int r = 0; r < 10; ++r) {
+        reinit_update(q, y, &st);
+        Slope s;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            s.p[k] = y.pg[k];
+            s.n[k] = y.ng[k];
+        }
+        int next; /* 1, 2, 3: the next state is that RK3 stage; 4: AB3 */
+        if (r == 1 || r == 4 || r == 7) {
+            k1 = s;
+            k2 = t0;
+            next = r == 7 ? 3 : 2;
+        } else if (r == 2 || r == 5) {
+            k2 = s;
+            next = 3;
+        } else if (r == 8) {
+            next = 4;
+        } else if (r == 9) {
+            out.put(2, y);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                x.pos[k] = y.pos[k];
+                x.nd[k] = y.nd[k];
+            }
+            x.c = y.c;
+            return;
+        } else {
+            /* 0, 3, 6: a run starts here */
+            if (r == 0) {
+                t0 = s;
+            } else {
+                RayC& o = r == 3 ? c : v;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    o.pos[k] = y.pos[k];
+                    o.nd[k] = y.nd[k];
+                }
+                o.c = y.c;
+                out.put(r == 3 ? 1 : 0, y);
+                if (r == 3) {
+                    sc = s;
+                    st_c = st;
+                } else {
+                    sv = s;
+                }
+                h = -q.dt;
+            }
+            b0 = s;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                bp[k] = y.pos[k];
+                bn[k] = y.nd[k];
+            }
+            next = 1;
+        }
+        if (next == 1) { /* ode_integ.cc:20-126 */
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                y.pos[k] = bp[k] + 0.5 * h * b0.p[k];
+                y.nd[k] = bn[k] + 0.5 * h * b0.n[k];
+            }
+        } else if (next == 2) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                y.pos[k] = bp[k] + h * (2.0 * k1.p[k] - b0.p[k]);
+                y.nd[k] = bn[k] + h * (2.0 * k1.n[k] - b0.n[k]);
+            }
+        } else if (next == 3) {
+            const double h6 = quot(h, Recip{6.0, 1.0 / 6.0});
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                y.pos[k] = bp[k] + h6 * (b0.p[k] + 4.0 * k1.p[k] + k2.p[k]);
+                y.nd[k] = bn[k] + h6 * (b0.n[k] + 4.0 * k1.n[k] + k2.n[k]);
+            }
+        } else { /* ode_integ.cc:131-186; sin(theta) of curr is its update's */
+            const double A2 = 23.0 / 12.0, A1 = 16.0 / 12.0, A0 = 5.0 / 12.0;
+            const double dt = q.dt;
+            double d[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) d[k] = dt * (A2 * sc.p[k] - A1 * sv.p[k] + A0 * s.p[k]);
+            const double e = c.pos[0] * d[1];
+            const double f = c.pos[0] * (st_c * d[2]);
+            y.dist = sqrt(d[0] * d[0] + e * e + f * f);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                y.pos[k] = c.pos[k] + d[k];
+                y.nd[k] = c.nd[k] + dt * (A2 * sc.n[k] - A1 * sv.n[k] + A0 * s.n[k]);
+            }
+        }
+    }
 }
 
 __device__ void record_reflection(const QueueDev& q, int64_t step, double t_old,
@@ -496,77 +590,90 @@ __device__ void record_reflection(const QueueDev& q, int64_t step, double t_old,
     q.refl[slot] = r;
 }
 
-/* reflection_model::surface_reflection (reflection_model.cc:187-243) */
-__device__ __noinline__ bool surface_local(const QueueDev& q, const FrontPtrs& C, RayLocal& L, int i, int64_t step,
-                              double t_old, int& seq) {
-    double c = L.c.c;
-    const double d = c * c * L.c.nd[0];
-    const double tw = (d == 0.0) ? 0.0 : -(L.c.pos[0] - q.R) / d;
-    double pos[3], nd[3];
-    collision_local(q, L, tw, pos, nd, &c);
-    const double n1 = L.c.nd[1], n2 = L.c.nd[2];
-    const double grazing = atan2(L.c.nd[0], sqrt(n1 * n1 + n2 * n2));
-    if (grazing <= 0.0) return false;
-    record_reflection(q, step, t_old, i, tw, grazing, c, pos, nd, 1, seq);
-    if (q.want_verbs)
-        build_eigenverb(q, C, i, step, t_old, tw, grazing, c, pos, nd, WQ3D_VERB_SURFACE, L.c.c, L.surface,
-                        L.bottom, seq);
-    ++seq;
-    const LossDev& Lo = q.oc.surf.loss;
-    double amp0 = 0.0, ph0 = 0.0;
-    if (Lo.kind != WQ3D_LOSS_ECKART) reflect_loss_scalar(Lo, grazing, &amp0, &ph0);
-    const double w2 = Lo.p[0] * Lo.p[0];
-    const double sg = sin(grazing);
-    for (int k = 0; k < q.nf; ++k) {
-        double a = amp0;
-        if (Lo.kind == WQ3D_LOSS_ECKART) {
-            const double x = q.freq[k] * w2 * sg;
-            a = 8.6e-9 * (x * x);
-        }
-        L.att[k] += a;
-        L.ph[k] -= M_PI;
-        L.phf[k] -= M_PI;
+/* one bounce's loss: what every frequency's attenuation and phase gain,
+ * or for a wind-driven surface (Eckart) the sine of the grazing angle */
+struct Loss {
+    double amp, ph, sin_grazing;
+    int eckart; /* 0, or the boundary (1 surface, 2 bottom) whose wind sets it */
+};
+
+__device__ __forceinline__ void bounce_loss(const LossDev& Lo, double grazing, int which, Loss& o) {
+    o.amp = o.ph = o.sin_grazing = 0.0;
+    o.eckart = 0;
+    if (Lo.kind == WQ3D_LOSS_ECKART) {
+        o.eckart = which;
+        o.sin_grazing = sin(grazing);
+    } else {
+        reflect_loss_scalar(Lo, grazing, &o.amp, &o.ph);
     }
-    nd[0] = -nd[0];
-    reinit_local(q, L, tw, pos, nd);
-    return true;
 }
 
-/* reflection_model::bottom_reflection (reflection_model.cc:33-182) */
-__device__ __noinline__ void bottom_local(const QueueDev& q, const FrontPtrs& C, RayLocal& L, int i, double depth,
-                             int64_t step, double t_old, int& seq, double* dl) {
+/* reflection_model::surface_reflection (reflection_model.cc:187-243) up to
+ * the re-initialisation, for a ray heading up (the reference's grazing angle
+ * is positive exactly when the curr direction's radial part is): collision
+ * time, point and reflected direction.  The angle itself is formed only for
+ * those who read it. */
+template <class Out>
+__device__ __forceinline__ void surface_bounce(const QueueDev& q, const FrontPtrs& C, const RayC& v, const RayC& cr,
+                                               const RayC& x, int i, int64_t step, double t_old, int surface,
+                                               int bottom, int& seq, double* tw_out, double* pos, double* nd,
+                                               Out& out) {
+    double c = cr.c;
+    const double d = c * c * cr.nd[0];
+    const double tw = (d == 0.0) ? 0.0 : -(cr.pos[0] - q.R) / d;
+    collision_rays(q, v, cr, x, tw, pos, nd, &c);
+    const LossDev& Lo = q.oc.surf.loss;
+    double grazing = 0.0;
+    if (q.want_refl || q.want_verbs || Lo.kind == WQ3D_LOSS_ECKART || Lo.kind == WQ3D_LOSS_RAYLEIGH) {
+        const double n1 = cr.nd[1], n2 = cr.nd[2];
+        grazing = atan2(cr.nd[0], sqrt(n1 * n1 + n2 * n2));
+    }
+    record_reflection(q, step, t_old, i, tw, grazing, c, pos, nd, 1, seq);
+    if (q.want_verbs)
+        build_eigenverb(q, C, i, step, t_old, tw, grazing, c, pos, nd, WQ3D_VERB_SURFACE, cr.c, surface, bottom, seq);
+    ++seq;
+    if (out.losses()) {
+        Loss l;
+        bounce_loss(Lo, grazing, 1, l);
+        l.ph = -M_PI;
+        out.add(l);
+    }
+    nd[0] = -nd[0];
+    *tw_out = tw;
+}
+
+/* reflection_model::bottom_reflection (reflection_model.cc:33-182) up to
+ * the re-initialisation */
+template <class Out>
+__device__ __forceinline__ void bottom_bounce(const QueueDev& q, const FrontPtrs& C, const RayC& v, const RayC& cr,
+                                              const RayC& x, int i, double depth, int64_t step, double t_old,
+                                              int surface, int bottom, int& seq, double* tw_out, double* position,
+                                              double* ndir, Out& out) {
     const BoundaryDev& B = q.oc.bot;
-    bool shallow = false;
-    double position[3] = {L.c.pos[0], L.c.pos[1], L.c.pos[2]};
-    double ndir[3] = {L.c.nd[0], L.c.nd[1], L.c.nd[2]};
-    double c = L.c.c;
+    double c = cr.c;
     double c2 = c * c;
     double nrm[3];
-    double bottom_rho = boundary_height_normal(B, position[1], position[2], nrm);
-    double height_water = position[0] - bottom_rho;
+    double bottom_rho = boundary_height_normal(B, cr.pos[1], cr.pos[2], nrm);
+    double height_water = cr.pos[0] - bottom_rho;
     const double TOO_SHALLOW = 300.0 * q.dt;
-    if ((q.R - bottom_rho) < TOO_SHALLOW) shallow = true;
-    double N;
+    const bool shallow = (q.R - bottom_rho) < TOO_SHALLOW;
     if (shallow) {
-        N = sqrt(nrm[1] * nrm[1] + nrm[2] * nrm[2]);
+        const double N = sqrt(nrm[1] * nrm[1] + nrm[2] * nrm[2]);
         nrm[0] = 0.0;
         nrm[1] = nrm[1] / N;
         nrm[2] = nrm[2] / N;
     }
-    ndir[0] = c2 * ndir[0];
-    ndir[1] = c2 * ndir[1];
-    ndir[2] = c2 * ndir[2];
-    double dot_full = nrm[0] * ndir[0] + nrm[1] * ndir[1] + nrm[2] * ndir[2];
+    double dot_full = nrm[0] * (c2 * cr.nd[0]) + nrm[1] * (c2 * cr.nd[1]) + nrm[2] * (c2 * cr.nd[2]);
     const double MIN_REFLECT = 6.0;
     double max_dot = -fmax(MIN_REFLECT, (height_water + depth) * nrm[0]);
     if (dot_full >= max_dot) dot_full = max_dot;
     const double dot_water = -height_water * nrm[0];
     const double time_water = fmax(0.0, dot_water / dot_full);
 
-    collision_local(q, L, time_water, position, ndir, &c);
+    collision_rays(q, v, cr, x, time_water, position, ndir, &c);
     bottom_rho = boundary_height_normal(B, position[1], position[2], nrm);
     if (shallow) {
-        N = sqrt(nrm[1] * nrm[1] + nrm[2] * nrm[2]);
+        const double N = sqrt(nrm[1] * nrm[1] + nrm[2] * nrm[2]);
         nrm[0] = 0.0;
         nrm[1] = nrm[1] / N;
         nrm[2] = nrm[2] / N;
@@ -581,61 +688,94 @@ __device__ __noinline__ void bottom_local(const QueueDev& q, const FrontPtrs& C,
     if (dot_full >= max_dot) dot_full = max_dot;
 
     double grazing;
-    if (dot_full / c >= 1.0) {
+    const double sine = dot_full / c;
+    if (sine >= 1.0) {
         grazing = -M_PI_2;
-    } else if (dot_full / c <= -1.0) {
+    } else if (sine <= -1.0) {
         grazing = M_PI_2;
     } else {
-        grazing = asin(-dot_full / c);
+        grazing = asin(-sine);
     }
     record_reflection(q, step, t_old, i, time_water, grazing, c, position, ndir, 0, seq);
     if (q.want_verbs)
-        build_eigenverb(q, C, i, step, t_old, time_water, grazing, c, position, ndir, WQ3D_VERB_BOTTOM, L.c.c,
-                        L.surface, L.bottom, seq);
+        build_eigenverb(q, C, i, step, t_old, time_water, grazing, c, position, ndir, WQ3D_VERB_BOTTOM, cr.c, surface,
+                        bottom, seq);
     ++seq;
-
-    const LossDev& Lo = B.loss;
-    double amp0 = 0.0, ph0 = 0.0;
-    if (Lo.kind != WQ3D_LOSS_ECKART) reflect_loss_scalar(Lo, grazing, &amp0, &ph0);
-    if (q.sens) {
-        double g[3];
-        reflect_loss_rayleigh_grad(Lo, grazing, g);
-        for (int j = 0; j < 3; ++j) dl[j] += g[j];
-    }
-    const double w2 = Lo.p[0] * Lo.p[0];
-    const double sgz = sin(grazing);
-    for (int k = 0; k < q.nf; ++k) {
-        double a = amp0, p = ph0;
-        if (Lo.kind == WQ3D_LOSS_ECKART) {
-            const double x = q.freq[k] * w2 * sgz;
-            a = 8.6e-9 * (x * x);
-            p = M_PI;
+    if (out.losses()) {
+        Loss l;
+        bounce_loss(B.loss, grazing, 2, l);
+        if (B.loss.kind == WQ3D_LOSS_ECKART) l.ph = M_PI;
+        out.add(l);
+        if (q.sens) {
+            double g[3];
+            reflect_loss_rayleigh_grad(B.loss, grazing, g);
+            out.tangents(g);
         }
-        L.att[k] += a;
-        L.ph[k] += p;
-        L.phf[k] += p;
     }
     dot_full *= 2.0;
     ndir[0] = ndir[0] - dot_full * nrm[0];
     ndir[1] = ndir[1] - dot_full * nrm[1];
     ndir[2] = ndir[2] - dot_full * nrm[2];
-    N = sqrt(ndir[0] * ndir[0] + ndir[1] * ndir[1] + ndir[2] * ndir[2]) * c;
-    ndir[0] = ndir[0] / N;
-    ndir[1] = ndir[1] / N;
-    ndir[2] = ndir[2] / N;
-    reinit_local(q, L, time_water, position, ndir);
+    const double N = sqrt(ndir[0] * ndir[0] + ndir[1] * ndir[1] + ndir[2] * ndir[2]) * c;
+    if (divisor_ok(N) && dividend_ok(ndir[0]) && dividend_ok(ndir[1]) && dividend_ok(ndir[2])) {
+        const Recip r = recip(N);
+        ndir[0] = quot(ndir[0], r);
+        ndir[1] = quot(ndir[1], r);
+        ndir[2] = quot(ndir[2], r);
+    } else {
+        ndir[0] = ndir[0] / N;
+        ndir[1] = ndir[1] / N;
+        ndir[2] = ndir[2] / N;
+    }
+    *tw_out = time_water;
+}
+
+/* The reference's detect_reflections for one ray (wave_queue.cc:197-256):
+ * volume layers, then the surface / bottom chain, volume layers after each
+ * reflection.  A ray tries the surface first, else the bottom, and after a
+ * bounce the other boundary, until it meets none; out.stop(n) may end the
+ * chain after n bounces.  v, c, x: the ray's prev, curr and next states,
+ * replaced by the reflected ones. */
+template <class Out>
+__device__ __forceinline__ void bounce_chain(const QueueDev& q, const FrontPtrs& C, int i, int64_t step, double t_old,
+                                             RayC& v, RayC& c, RayC& x, int& surface, int& bottom, Out& out) {
+    const bool vol = q.want_verbs && q.oc.nvol > 0;
+    int seq = 0; /* orders the ray's events */
+    int last = -1; /* 0 the surface, 1 the bottom */
+    if (vol) volume_scatter(q, C, i, step, t_old, v, c, x, surface, bottom, seq);
+#pragma unroll 1
+    for (int n = 0;; ++n) {
+        if (n > 0 && out.stop(n)) return;
+        const bool surf = last != 0 && x.pos[0] - q.R > 0.0 && !(c.nd[0] <= 0.0);
+        double depth = 0.0;
+        if (!surf) {
+            if (last == 1) return;
+            depth = boundary_height(q.oc.bot, x.pos[1], x.pos[2]) - x.pos[0];
+            if (!(depth > 0.0)) return;
+        }
+        double tw, pos[3], nd[3];
+        if (surf)
+            surface_bounce(q, C, v, c, x, i, step, t_old, surface, bottom, seq, &tw, pos, nd, out);
+        else
+            bottom_bounce(q, C, v, c, x, i, depth, step, t_old, surface, bottom, seq, &tw, pos, nd, out);
+        reinit_ray(q, v, c, x, tw, pos, nd, out);
+        out.bounced(!surf);
+        if (surf)
+            ++surface;
+        else
+            ++bottom;
+        last = surf ? 0 : 1;
+        if (vol) volume_scatter(q, C, i, step, t_old, v, c, x, surface, bottom, seq);
+    }
 }
 
 /* whether the "next" ray reflects at the start of the following step:
  * 1 = surface if above the surface and heading up (surface_reflection's
- * grazing > 0), else 2 = bottom if below the bottom (wave_queue.cc:222-256) */
+ * grazing > 0, which is the sign of the direction's radial part), else 2 = bottom if below the bottom (wave_queue.cc:222-256) */
 __device__ __forceinline__ uint8_t reflect_decision(const QueueDev& q,
                                                     const double* xpos,
                                                     const double* cnd) {
-    if (xpos[0] - q.R > 0.0) {
-        const double grazing = atan2(cnd[0], sqrt(cnd[1] * cnd[1] + cnd[2] * cnd[2]));
-        if (grazing > 0.0) return 1;
-    }
+    if (xpos[0] - q.R > 0.0 && cnd[0] > 0.0) return 1;
     const double h = boundary_height(q.oc.bot, xpos[1], xpos[2]);
     return (h - xpos[0] > 0.0) ? 2 : 0;
 }
@@ -795,87 +935,85 @@ __global__ void __launch_bounds__(128) k_startup(__grid_constant__ const QueueDe
 /* then every ray advances                                             */
 /* ------------------------------------------------------------------ */
 
-/* The reflection chain of ray i at the start of step s (wave_queue.cc:
- * 197-256) on L: the ray's prev, curr and next states, counts and next-front
- * losses before the step's reflections.  The result goes to slot w of set
- * shadow_set(s); k_advance of step s takes it from there.  The caustic
- * hand-off from the D/E neighbour below (wave_queue.cc:274-292), which the
- * reference runs before the ray reflects, is decided by k_advance of step
- * s, when that neighbour's next front is complete; the slot carries the
- * phases both without and with its -pi/2 shift. */
-__device__ __forceinline__ void reflect_chain_body(const QueueDev& q, int64_t s, int i, uint32_t w,
-                                                   RayLocal& L, double t_old) {
+/* The shadow slot of a reflecting ray as its chain fills it (see
+ * shadow_stride).  The frequencies' losses are kept per bounce and applied
+ * once, at the end. */
+struct SlotOut {
+    const QueueDev& q;
+    double* sh;
+    double dl[3];
+    int n;
+    Loss loss[MAX_BOUNCE + 2];
+    __device__ SlotOut(const QueueDev& q_, double* sh_) : q(q_), sh(sh_), dl{0.0, 0.0, 0.0}, n(0) {}
+    __device__ void put(int which, const RayS& y) { ray_to(sh + 17 * which, y); }
+    __device__ bool losses() const { return true; }
+    __device__ void add(const Loss& l) { loss[n++] = l; }
+    __device__ void tangents(const double* g) {
+        for (int j = 0; j < 3; ++j) dl[j] += g[j];
+    }
+    __device__ void bounced(bool) {}
+    __device__ bool stop(int bounces) {
+        if (bounces <= MAX_BOUNCE) return false;
+        set_err(q, ERR_BOUNCE_LIMIT);
+        return true;
+    }
+    /* attenuation and phase of frequency f before the reflections */
+    __device__ void apply(int f, double att, double ph) {
+        double phf = ph - M_PI_2;
+        for (int k = 0; k < n; ++k) {
+            double a = loss[k].amp;
+            if (loss[k].eckart) {
+                const LossDev& Lo = loss[k].eckart == 1 ? q.oc.surf.loss : q.oc.bot.loss;
+                const double x = q.freq[f] * (Lo.p[0] * Lo.p[0]) * loss[k].sin_grazing;
+                a = 8.6e-9 * (x * x);
+            }
+            att += a;
+            ph += loss[k].ph;
+            phf += loss[k].ph;
+        }
+        sh[51 + f] = att;
+        sh[51 + q.nf + f] = ph;
+        sh[54 + 2 * q.nf + f] = phf;
+    }
+};
+
+/* The reflection chain of ray i at the start of step s on the ray's prev,
+ * curr and next states v, c, x; surface, bottom, caustic: its counts, atten
+ * and phase: its next-front losses ([f][n]), all before the step's
+ * reflections.  The result goes to slot w of set shadow_set(s); k_advance of
+ * step s takes it from there.  (The launch that listed the ray made the
+ * chain's first test on the same values, so at least one bounce fills the
+ * slot.)  The caustic hand-off from the D/E neighbour below (wave_queue.cc:
+ * 274-292), which the reference runs before the ray reflects, is decided by
+ * k_advance of step s, when that neighbour's next front is complete; the
+ * slot carries the phases both without and with its -pi/2 shift. */
+__device__ __forceinline__ void reflect_chain_body(const QueueDev& q, int64_t s, int i, uint32_t w, RayC& v, RayC& c,
+                                                   RayC& x, int surface, int bottom, int caustic,
+                                                   const double* atten, const double* phase, double t_old) {
     Roles R;
     roles_at(q, s, R);
-    for (int f = 0; f < q.nf; ++f) L.phf[f] = L.ph[f] - M_PI_2;
-    /* the reference's detect_reflections for this ray: volume layers,
-     * then the surface / bottom chain, volume layers after each
-     * reflection (wave_queue.cc:202-256); seq orders the ray's events */
-    const bool vol = q.want_verbs && q.oc.nvol > 0;
-    double dl[3] = {0.0, 0.0, 0.0};
-    bool reflected = false;
-    int seq = 0;
-    int next_try = -1; /* 0: try bottom next, 1: try surface next */
-    if (vol) volume_scatter(q, *R.C, i, s + 1, t_old, L.v, L.c, L.x, L.surface, L.bottom, seq);
-    if (L.x.pos[0] - q.R > 0.0 && surface_local(q, *R.C, L, i, s + 1, t_old, seq)) {
-        L.surface += 1;
-        reflected = true;
-        next_try = 0;
-    } else {
-        const double depth = boundary_height(q.oc.bot, L.x.pos[1], L.x.pos[2]) - L.x.pos[0];
-        if (depth > 0.0) {
-            bottom_local(q, *R.C, L, i, depth, s + 1, t_old, seq, dl);
-            L.bottom += 1;
-            reflected = true;
-            next_try = 1;
-        }
-    }
-    if (reflected) {
-        if (vol) volume_scatter(q, *R.C, i, s + 1, t_old, L.v, L.c, L.x, L.surface, L.bottom, seq);
-        int it = 0;
-        for (; it < MAX_BOUNCE; ++it) {
-            if (next_try == 0) {
-                const double depth = boundary_height(q.oc.bot, L.x.pos[1], L.x.pos[2]) - L.x.pos[0];
-                if (!(depth > 0.0)) break;
-                bottom_local(q, *R.C, L, i, depth, s + 1, t_old, seq, dl);
-                L.bottom += 1;
-                next_try = 1;
-            } else {
-                if (!(L.x.pos[0] - q.R > 0.0 && surface_local(q, *R.C, L, i, s + 1, t_old, seq))) break;
-                L.surface += 1;
-                next_try = 0;
-            }
-            if (vol) volume_scatter(q, *R.C, i, s + 1, t_old, L.v, L.c, L.x, L.surface, L.bottom, seq);
-        }
-        if (it == MAX_BOUNCE) set_err(q, ERR_BOUNCE_LIMIT);
-    }
     const int set = shadow_set(s);
-    const size_t stride = shadow_stride(q);
-    double* sh = q.shadow[set] + (size_t)w * stride;
-    ray_to(sh, L.v);
-    ray_to(sh + 17, L.c);
-    ray_to(sh + 34, L.x);
-    for (int f = 0; f < q.nf; ++f) {
-        sh[51 + f] = L.att[f];
-        sh[51 + q.nf + f] = L.ph[f];
-        sh[54 + 2 * q.nf + f] = L.phf[f];
-    }
+    SlotOut out(q, q.shadow[set] + (size_t)w * shadow_stride(q));
+    bounce_chain(q, *R.C, i, s + 1, t_old, v, c, x, surface, bottom, out);
+    for (int f = 0; f < q.nf; ++f) out.apply(f, atten[(size_t)f * q.n + i], phase[(size_t)f * q.n + i]);
     /* the next front's loss tangents take this step's bottom bounces
      * when k_commit applies the slot; the previous step's eigenray
      * construction may still be reading them */
     if (q.sens)
-        for (int j = 0; j < 3; ++j) sh[51 + 2 * q.nf + j] = dl[j];
-    q.shadow_cnt[set][3 * (size_t)w] = L.surface;
-    q.shadow_cnt[set][3 * (size_t)w + 1] = L.bottom;
-    q.shadow_cnt[set][3 * (size_t)w + 2] = L.caustic;
+        for (int j = 0; j < 3; ++j) out.sh[51 + 2 * q.nf + j] = out.dl[j];
+    q.shadow_cnt[set][3 * (size_t)w] = surface;
+    q.shadow_cnt[set][3 * (size_t)w + 1] = bottom;
+    q.shadow_cnt[set][3 * (size_t)w + 2] = caustic;
     q.shadow_slot[set][i] = (int32_t)w;
 }
 
 /* out of line for the inline schedule's advance, whose other rays need
  * none of its registers */
-__device__ __noinline__ void reflect_chain(const QueueDev& q, int64_t s, int i, uint32_t w, RayLocal& L,
-                                           double t_old) {
-    reflect_chain_body(q, s, i, w, L, t_old);
+__device__ __noinline__ void reflect_chain(const QueueDev& q, int64_t s, int i, uint32_t w, const RayC& v,
+                                           const RayC& c, const RayC& x, int surface, int bottom, int caustic,
+                                           const double* atten, const double* phase, double t_old) {
+    RayC a = v, b = c, d = x;
+    reflect_chain_body(q, s, i, w, a, b, d, surface, bottom, caustic, atten, phase, t_old);
 }
 
 /* Reflecting rays of step s listed by the launch that produced the "next"
@@ -897,24 +1035,19 @@ __global__ void __launch_bounds__(64) k_reflect(__grid_constant__ const QueueDev
         const uint32_t w = ww < nsurf ? ww : (uint32_t)q.n - 1 - (ww - nsurf);
         const int i = (int)work[w];
         WQ_CHECKED_OR(q, i >= 0 && i < q.n, continue);
-        RayLocal L;
-        {
-            /* the fronts are read-only here */
-            RayS v, c, x;
-            load_prev_curr(q, s, R, i, v, c);
-            load_ray_ro(*R.X, i, x);
-            L.v = v;
-            L.c = c;
-            L.x = x;
-            L.surface = __ldg(R.X->surface + i);
-            L.bottom = __ldg(R.X->bottom + i);
-            L.caustic = __ldg(R.X->caustic + i);
+        /* the fronts are read-only here */
+        RayC v, c, x;
+        const double* sp = prev_step_slot(q, s, i);
+        if (sp) {
+            rayc_from(sp + 17, v);
+            rayc_from(sp + 34, c);
+        } else {
+            load_rayc(*R.V, i, v);
+            load_rayc(*R.C, i, c);
         }
-        for (int f = 0; f < q.nf; ++f) {
-            L.att[f] = __ldg(R.X->atten + (size_t)f * q.n + i);
-            L.ph[f] = __ldg(R.X->phase + (size_t)f * q.n + i);
-        }
-        reflect_chain_body(q, s, i, w, L, t_old);
+        load_rayc(*R.X, i, x);
+        reflect_chain_body(q, s, i, w, v, c, x, __ldg(R.X->surface + i), __ldg(R.X->bottom + i),
+                           __ldg(R.X->caustic + i), R.X->atten, R.X->phase, t_old);
     }
     /* the last block to finish empties this step's worklist, which the
      * advance of step s+1 refills (every block has read the count by then;
@@ -936,14 +1069,11 @@ __global__ void __launch_bounds__(64) k_reflect(__grid_constant__ const QueueDev
  * becomes "curr" (wave_front.cc:184-216; reflecting neighbours are read
  * from their shadow slots), the rotation, AB3 and update of the new front
  * (wave_queue.cc:162-183), and the reflection decision of the next step. */
-/* five blocks per SM for the analytic build (96 registers, spills to L1
- * that cost less than the lost occupancy); the gridded build calls the
- * out-of-line grid interpolation and keeps its full register budget */
-#if WQ3D_WITH_GRID
-#define WQ_ADVANCE_BOUNDS __launch_bounds__(128)
-#else
+/* Five blocks per SM (96 registers, spills to L1 that cost less than the
+ * lost occupancy): the advance waits for memory.  Reverberation workload
+ * (651,781 rays, 32 frequencies): 322 us at five, 352 at four, 408 at three,
+ * 519 at two blocks; fans that do not fill the GPU do not care. */
 #define WQ_ADVANCE_BOUNDS __launch_bounds__(128, 5)
-#endif
 template <bool INLINE>
 __device__ __forceinline__ void advance_body(const QueueDev& q, int k) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1155,32 +1285,24 @@ __device__ __forceinline__ void advance_body(const QueueDev& q, int k) {
     /* the reflections of step s+1 right here: this ray's prev and curr
      * states at step s+1 are its curr and next at step s, its next the
      * front just written (read back by this thread) */
-    RayLocal L;
+    RayC v, c;
     if (refl) {
-        ray_from(sh + 17, L.v);
-        ray_from(sh + 34, L.c);
+        rayc_from(sh + 17, v);
+        rayc_from(sh + 34, c);
     } else {
         const double* sp = prev_step_slot(q, s, i);
         if (sp)
-            ray_from(sp + 34, L.v);
+            rayc_from(sp + 34, v);
         else
-            load_ray_ro(*R.C, i, L.v);
-        load_ray_ro(*R.X, i, L.c);
-    }
-    L.x = y3;
-    L.surface = sf;
-    L.bottom = bt;
-    L.caustic = cs;
-    for (int f = 0; f < q.nf; ++f) {
-        L.att[f] = P.atten[(size_t)f * q.n + i];
-        L.ph[f] = P.phase[(size_t)f * q.n + i];
+            load_rayc(*R.C, i, v);
+        load_rayc(*R.X, i, c);
     }
     const uint32_t w = atomicAdd(q.n_slot + shadow_set(s + 1), 1u);
     if (w >= (uint32_t)q.n) {
         set_err(q, ERR_SLOT_OVERFLOW);
         return;
     }
-    reflect_chain(q, s + 1, i, w, L, q.d_times[k + 1]);
+    reflect_chain(q, s + 1, i, w, v, c, rayc_of(y3), sf, bt, cs, P.atten, P.phase, q.d_times[k + 1]);
 }
 
 /* the side schedule: the reflecting rays of step s+1 go to the worklist
@@ -1191,7 +1313,7 @@ __global__ void WQ_ADVANCE_BOUNDS k_advance(__grid_constant__ const QueueDev q, 
 
 /* the inline schedule: each thread runs step s+1's reflection chain of
  * its ray itself */
-__global__ void WQ_ADVANCE_BOUNDS k_advance_inline(__grid_constant__ const QueueDev q, int k) {
+__global__ void __launch_bounds__(128, 2) k_advance_inline(__grid_constant__ const QueueDev q, int k) {
     advance_body<true>(q, k);
 }
 
@@ -1269,10 +1391,10 @@ __global__ void __launch_bounds__(128) k_volume(__grid_constant__ const QueueDev
     bool cross = false;
     for (int v = 0; v < q.oc.nvol; ++v) cross |= (q.oc.vol_rho[v] - rx) * (q.oc.vol_rho[v] - rc) < 0;
     if (!cross) return;
-    RayS y0, y1, y2;
-    load_ray(*R.V, i, y0);
-    load_ray(*R.C, i, y1);
-    load_ray(*R.X, i, y2);
+    RayC y0, y1, y2;
+    load_rayc(*R.V, i, y0);
+    load_rayc(*R.C, i, y1);
+    load_rayc(*R.X, i, y2);
     int seq = 0;
     volume_scatter(q, *R.C, i, s + 1, q.d_times[k], y0, y1, y2, R.C->surface[i], R.C->bottom[i], seq);
 }
