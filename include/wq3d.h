@@ -409,8 +409,10 @@ int wq3d_queue_destroy(wq3d_queue* q);
  * of the same device, fan, frequency, target and eigenray-capacity shape
  * instead of allocating: a create-run-destroy loop then allocates and
  * instantiates its graphs once.  Results are those of a fresh queue.
- * max_queues = 0 frees the cached queues and turns the cache off.  The
- * reference has no counterpart (each wave_queue owns its fronts). */
+ * Other destroyed queues leave their streams and events (32 at most) and
+ * their device memory (up to an eighth of the device's) to later queues.
+ * max_queues = 0 frees all of that and turns the cache off.  The reference
+ * has no counterpart (each wave_queue owns its fronts). */
 int wq3d_set_queue_cache(size_t max_queues);
 
 /* Sensitivity mode (call before the first step): every eigenray also

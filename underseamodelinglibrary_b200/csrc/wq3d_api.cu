@@ -141,6 +141,62 @@ struct DeviceGuard {
     }
 };
 
+/* Device memory of queues.  A program that makes, runs and drops queues paid
+ * cudaMalloc and cudaFree (which wait for the whole device) some forty times
+ * a queue: 20 ms to over a second for the reverberation workload's 5 GB.
+ * Each device has one pool instead, from which allocation and release are
+ * ordered on the queue's stream.  It keeps up to an eighth of the device's
+ * memory between queues; wq3d_set_queue_cache(0) gives that back. */
+constexpr int MAX_POOL_DEVICES = 64;
+std::mutex g_pool_mu;
+cudaMemPool_t g_pool[MAX_POOL_DEVICES] = {};
+
+cudaError_t device_pool(int device, cudaMemPool_t* out) {
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    if (device < 0 || device >= MAX_POOL_DEVICES) return cudaErrorInvalidDevice;
+    if (!g_pool[device]) {
+        cudaMemPoolProps props;
+        std::memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.handleTypes = cudaMemHandleTypeNone;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaMemPool_t pool = nullptr;
+        cudaError_t e = cudaMemPoolCreate(&pool, &props);
+        if (e != cudaSuccess) return e;
+        size_t free_b = 0, total_b = 0;
+        e = cudaMemGetInfo(&free_b, &total_b);
+        uint64_t keep = total_b / 8;
+        if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e != cudaSuccess) {
+            cudaMemPoolDestroy(pool);
+            return e;
+        }
+        g_pool[device] = pool;
+    }
+    *out = g_pool[device];
+    return cudaSuccess;
+}
+
+/* bytes that the device's pool holds and no queue uses */
+size_t pool_idle_bytes(int device) {
+    cudaMemPool_t pool;
+    uint64_t held = 0, used = 0;
+    if (device_pool(device, &pool) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return held > used ? (size_t)(held - used) : 0;
+}
+
+void trim_pools() {
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    for (auto& pool : g_pool)
+        if (pool) cudaMemPoolTrimTo(pool, 0);
+}
+
 }  // namespace
 
 struct wq3d_ocean {
@@ -251,6 +307,8 @@ int make_grid(wq3d_ocean* o, const wq3d_grid_desc& d, int max_dims, GridDev* hg,
     }
     if (!rc && hg->unrolled == GRID_PCHIP0) rc = up(pch.data(), pch.size(), &dg->ax[0].pch);
     if (!rc) rc = up(hg->data, total, &dg->data);
+    /* a queue's streams do not wait for the default stream's copies */
+    if (!rc) WQ_CK(cudaStreamSynchronize(cudaStreamLegacy));
     return rc;
 }
 
@@ -372,10 +430,6 @@ void cpa_targets(const std::vector<double>& r, const std::vector<double>& th, co
  * of 4096 (reverberation workload), 10 for 34 of 100 (Munk workload).  The
  * steep bands, which keep the most, come first. */
 constexpr int CPA_PARTS = 8;
-
-/* the most patches that a fan of this size can have: a band of r rows has
- * at most naz r / 32 + 1 */
-size_t cpa_patch_limit(size_t nde, size_t naz) { return CPA_PARTS * (naz * (nde + 31) / 32 + nde + 1); }
 
 void cpa_patches(const std::vector<double>& de, const std::vector<double>& az, size_t nt,
                  std::vector<CpaPatch>* out) {
@@ -502,19 +556,90 @@ struct PendingRays {
     }
 };
 
-struct wq3d_queue {
-    int device = 0;
+/* A queue's streams, events and pinned words: nothing in them depends on
+ * its shape, so destroyed queues leave them to later ones (rt_take, rt_give;
+ * making them took longer than a small queue's start-up). */
+struct QueueRt {
+    int device = -1;
     cudaStream_t stream = nullptr;
     cudaStream_t side = nullptr;
     cudaStream_t eig = nullptr; /* k_commit and the eigenray construction */
     cudaStream_t adv = nullptr; /* k_advance, checkpoints, volume eigenverbs */
-    cudaEvent_t start_ev = nullptr;
+    cudaStream_t copy = nullptr; /* record read-back */
+    cudaEvent_t start_ev = nullptr, eig_end = nullptr, ev_begin = nullptr, ev_end = nullptr;
+    cudaEvent_t done_ev[2] = {nullptr, nullptr}; /* a chunk's counters are on the host */
     std::vector<cudaEvent_t> fork_ev, join_ev;
     std::vector<cudaEvent_t> adv_ev, com_ev, cpa_ev; /* per step of a chunk */
-    cudaEvent_t eig_end = nullptr;
+    void* pinned = nullptr;
+
+    void destroy() {
+        for (auto* v : {&fork_ev, &join_ev, &adv_ev, &com_ev, &cpa_ev})
+            for (auto e : *v)
+                if (e) cudaEventDestroy(e);
+        for (auto e : {start_ev, eig_end, ev_begin, ev_end, done_ev[0], done_ev[1]})
+            if (e) cudaEventDestroy(e);
+        for (auto s : {copy, adv, eig, side, stream})
+            if (s) cudaStreamDestroy(s);
+        if (pinned) cudaFreeHost(pinned);
+        *this = QueueRt();
+    }
+    int make(int dev, int chunk, size_t pinned_bytes) {
+        device = dev;
+        /* the reflections are the longest chain of a step (one thread per
+         * reflecting ray): their blocks go first when SMs free up */
+        int prio_low = 0, prio_high = 0;
+        if (cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high) != cudaSuccess) prio_high = 0;
+        WQ_CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+        WQ_CK(cudaStreamCreateWithPriority(&side, cudaStreamNonBlocking, prio_high));
+        for (auto* st : {&eig, &adv, &copy}) WQ_CK(cudaStreamCreateWithFlags(st, cudaStreamNonBlocking));
+        WQ_CK(cudaEventCreate(&ev_begin));
+        WQ_CK(cudaEventCreate(&ev_end));
+        for (auto* e : {&start_ev, &eig_end, &done_ev[0], &done_ev[1]})
+            WQ_CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+        for (auto* v : {&fork_ev, &join_ev, &adv_ev, &com_ev, &cpa_ev}) {
+            v->assign(chunk, nullptr);
+            for (auto& e : *v) WQ_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        }
+        if (cudaMallocHost(&pinned, pinned_bytes) != cudaSuccess)
+            return fail(WQ3D_ERR_NOMEM, "cudaMallocHost failed");
+        return WQ3D_OK;
+    }
+};
+
+constexpr size_t RT_KEPT = 32; /* bundles kept for later queues */
+std::mutex g_rt_mu;
+std::vector<QueueRt> g_rt;
+bool g_rt_on = true; /* off while wq3d_set_queue_cache(0) holds */
+
+bool rt_take(int device, QueueRt* out) {
+    std::lock_guard<std::mutex> lock(g_rt_mu);
+    for (size_t k = g_rt.size(); k-- > 0;)
+        if (g_rt[k].device == device) {
+            *out = g_rt[k];
+            g_rt.erase(g_rt.begin() + k);
+            return true;
+        }
+    return false;
+}
+
+/* takes an idle bundle; destroys it when enough are kept */
+void rt_give(QueueRt& rt) {
+    {
+        std::lock_guard<std::mutex> lock(g_rt_mu);
+        if (g_rt_on && g_rt.size() < RT_KEPT) {
+            g_rt.push_back(rt);
+            rt = QueueRt();
+            return;
+        }
+    }
+    rt.destroy();
+}
+
+struct wq3d_queue : QueueRt {
     QueueDev h{};
     std::vector<void*> allocs;
-    void* pinned = nullptr;
+    char* inputs = nullptr; /* every uploaded array, one block */
+    size_t inputs_cap = 0;
     /* per result set: chunk base step, chunk times, counters read back
      * (n_rec, n_refl, err, -, work lists, n_done, -, n_verb); d_counts also
      * holds the bottom work lists (9, 10), the adjoint's mark and entry
@@ -532,6 +657,7 @@ struct wq3d_queue {
      * reflections] */
     cudaGraphExec_t graph[2][2][2] = {};
     bool graph_failed[2][2][2] = {};
+    int graph_uses[2][2][2] = {}; /* chunks launched without it */
     int64_t graph_launches[2][2][2] = {}; /* kernels in each graph */
     /* Reflection schedule (wq3d_queue_set_reflect_schedule).  Under
      * WQ3D_REFLECT_AUTO a queue run alone follows its shape's plan
@@ -559,8 +685,6 @@ struct wq3d_queue {
         double* verb_power = nullptr;
     } set1;
     bool have_set1 = false;
-    cudaEvent_t done_ev[2] = {nullptr, nullptr}; /* a chunk's counters are on the host */
-    cudaStream_t copy = nullptr;                 /* record read-back */
     /* delivered state (time(), steps()) and launched-through state */
     double time = 0.0;
     int64_t steps = 0;
@@ -580,7 +704,6 @@ struct wq3d_queue {
     bool timing = false;
     std::vector<cudaEvent_t> events;
     double ms_step = 0.0, ms_cpa = 0.0, ms_eig = 0.0, ms_total = 0.0, ms_refl = 0.0;
-    cudaEvent_t ev_begin = nullptr, ev_end = nullptr;
     int64_t launches = 0;
     /* the stepping kernels' build: "gridded" when the ocean has a grid */
     bool gridded = false;
@@ -590,10 +713,6 @@ struct wq3d_queue {
     /* eigenverb counting sink (wq3d_queue_count_eigenverbs) */
     bool count_verbs = false;
     uint64_t verb_counts[2 + 2 * WQ3D_MAX_VOLUME] = {0};
-    /* set while wq3d_queue_create re-initialises a queue taken from the
-     * cache of destroyed queues: uploads then copy into the buffers the
-     * queue already has */
-    bool reuse = false;
     char* ring = nullptr;   /* the wavefront ring's allocation */
     size_t ring_bytes = 0;
     /* adjoint workspace (wq3d_queue_adjoint), made on first use */
@@ -624,6 +743,7 @@ struct wq3d_queue {
                     if (graph[p][t][m]) cudaGraphExecDestroy(graph[p][t][m]);
                     graph[p][t][m] = nullptr;
                     graph_failed[p][t][m] = false;
+                    graph_uses[p][t][m] = 0;
                 }
     }
 
@@ -648,26 +768,16 @@ struct wq3d_queue {
         if (have_set1) return true;
         const size_t nf = (size_t)h.nf;
         ResultSet s;
-        std::vector<void*> got;
-        auto take = [&](auto** out, size_t count) {
-            void* p = nullptr;
-            if (cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(**out)) != cudaSuccess) {
-                cudaGetLastError();
-                return false;
-            }
-            got.push_back(p);
-            *out = static_cast<std::remove_reference_t<decltype(*out)>>(p);
-            return true;
-        };
-        bool ok = take(&s.rec, h.cap_rec) && take(&s.rec_inten, (size_t)h.cap_rec * nf) &&
-                  take(&s.rec_phase, (size_t)h.cap_rec * nf) && take(&s.refl, h.cap_refl) &&
-                  (!h.sens || take(&s.rec_sens, (size_t)h.cap_rec * 3)) &&
-                  (!h.verb || (take(&s.verb, h.cap_verb) && take(&s.verb_power, (size_t)h.cap_verb * nf)));
+        const size_t before = allocs.size();
+        bool ok = !alloc(&s.rec, h.cap_rec) && !alloc(&s.rec_inten, (size_t)h.cap_rec * nf) &&
+                  !alloc(&s.rec_phase, (size_t)h.cap_rec * nf) && !alloc(&s.refl, h.cap_refl) &&
+                  (!h.sens || !alloc(&s.rec_sens, (size_t)h.cap_rec * 3)) &&
+                  (!h.verb || (!alloc(&s.verb, h.cap_verb) && !alloc(&s.verb_power, (size_t)h.cap_verb * nf)));
         if (!ok) {
-            for (void* p : got) cudaFree(p);
+            cudaGetLastError();
+            while (allocs.size() > before) release(allocs.back());
             return false;
         }
-        allocs.insert(allocs.end(), got.begin(), got.end());
         set1 = s;
         have_set1 = true;
         return true;
@@ -679,7 +789,7 @@ struct wq3d_queue {
         if (!p) return;
         auto it = std::find(allocs.begin(), allocs.end(), p);
         if (it != allocs.end()) allocs.erase(it);
-        cudaFree(p);
+        cudaFreeAsync(p, stream);
     }
 
     /* A record buffer's capacity for "need" records of rec_bytes each: at
@@ -687,6 +797,7 @@ struct wq3d_queue {
     int record_capacity(size_t need, size_t rec_bytes, size_t* out) {
         size_t free_b = 0, total_b = 0;
         WQ_CK(cudaMemGetInfo(&free_b, &total_b));
+        free_b += pool_idle_bytes(device);
         const size_t limit = std::max<size_t>(4096, (free_b / 4) / rec_bytes);
         *out = std::min<size_t>({std::max<size_t>(need, 4096), limit, (size_t)UINT32_MAX / 2});
         return WQ3D_OK;
@@ -749,51 +860,65 @@ struct wq3d_queue {
     }
 
     ~wq3d_queue() {
+        for (auto st : {stream, side, eig, adv, copy})
+            if (st) cudaStreamSynchronize(st);
         drop_graph();
-        for (auto e : done_ev)
-            if (e) cudaEventDestroy(e);
         for (auto& pe : tune_ev)
             for (auto e : pe)
                 if (e) cudaEventDestroy(e);
-        if (copy) cudaStreamDestroy(copy);
         for (auto e : events)
             if (e) cudaEventDestroy(e);
-        for (auto e : fork_ev) cudaEventDestroy(e);
-        for (auto e : join_ev) cudaEventDestroy(e);
-        for (auto* v : {&adv_ev, &com_ev, &cpa_ev})
-            for (auto e : *v) cudaEventDestroy(e);
-        if (eig_end) cudaEventDestroy(eig_end);
-        if (start_ev) cudaEventDestroy(start_ev);
-        if (adv) cudaStreamDestroy(adv);
-        if (eig) cudaStreamDestroy(eig);
-        if (side) cudaStreamDestroy(side);
-        if (ev_begin) cudaEventDestroy(ev_begin);
-        if (ev_end) cudaEventDestroy(ev_end);
-        for (void* p : allocs) cudaFree(p);
-        if (pinned) cudaFreeHost(pinned);
-        if (stream) cudaStreamDestroy(stream);
+        for (void* p : allocs) cudaFreeAsync(p, stream);
+        if (stream) {
+            cudaStreamSynchronize(stream);
+            rt_give(*this);
+        }
     }
 
+    /* from the device's pool, ready for every stream when it returns */
     template <class T>
     int alloc(T** out, size_t count) {
         void* p = nullptr;
         const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
-        WQ_CK(cudaMalloc(&p, bytes));
+        cudaMemPool_t pool;
+        WQ_CK(device_pool(device, &pool));
+        cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool, stream);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            cudaMemPoolTrimTo(pool, 0);
+            e = cudaMallocFromPoolAsync(&p, bytes, pool, stream);
+        }
+        if (e != cudaSuccess) return fail(WQ3D_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
         allocs.push_back(p);
+        WQ_CK(cudaStreamSynchronize(stream));
         *out = static_cast<T*>(p);
         return WQ3D_OK;
     }
-    template <class T>
-    int upload(const T** out, const std::vector<T>& v) {
-        T* p = nullptr;
-        if (reuse && *out) {
-            p = const_cast<T*>(*out); /* same size: the cache key fixes every length */
-        } else {
-            int rc = alloc(&p, v.size());
-            if (rc) return rc;
+
+    /* The queue's input arrays, gathered on the host and sent as one copy
+     * on its stream (one cudaMemcpy each took 0.2 ms a queue). */
+    struct Inputs {
+        std::vector<char> bytes;
+        std::vector<std::pair<const void**, size_t>> at;
+        template <class T>
+        void add(const T** field, const std::vector<T>& v) {
+            const size_t off = (bytes.size() + 255) & ~size_t(255);
+            bytes.resize(off + std::max<size_t>(v.size(), 1) * sizeof(T), 0);
+            if (!v.empty()) std::memcpy(bytes.data() + off, v.data(), v.size() * sizeof(T));
+            at.push_back({reinterpret_cast<const void**>(field), off});
         }
-        if (!v.empty()) WQ_CK(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
-        *out = p;
+    };
+    int upload(const Inputs& in) {
+        if (in.bytes.size() > inputs_cap) {
+            if (inputs) release(inputs);
+            inputs = nullptr;
+            inputs_cap = 0;
+            const int rc = alloc(&inputs, in.bytes.size());
+            if (rc) return rc;
+            inputs_cap = in.bytes.size();
+        }
+        WQ_CK(cudaMemcpyAsync(inputs, in.bytes.data(), in.bytes.size(), cudaMemcpyHostToDevice, stream));
+        for (const auto& f : in.at) *f.first = inputs + f.second;
         return WQ3D_OK;
     }
 
@@ -1125,7 +1250,11 @@ struct wq3d_queue {
         chunk_trial[p] = trial;
         chunk_inl[p] = m;
         chunk_bucket[p] = bucket;
-        if (!timing && K == chunk) build_graph(p, tail, inl);
+        /* A graph pays from its second chunk on: capturing and instantiating
+         * one takes about as long as launching a chunk directly and replaying
+         * it, and a short run uses each once.  (A timed trial runs as later
+         * chunks will.) */
+        if (!timing && K == chunk && (trial || graph_uses[p][t][m]++ > 0)) build_graph(p, tail, inl);
         /* a trial times the chunk's device work only: its start is marked
          * after any graph building on the host */
         if (trial) {
@@ -1562,10 +1691,21 @@ int wq3d_set_queue_cache(size_t max_queues) {
             g_cache->erase(g_cache->begin());
         }
     }
+    std::vector<QueueRt> idle;
+    {
+        std::lock_guard<std::mutex> lock(g_rt_mu);
+        g_rt_on = max_queues > 0;
+        if (!g_rt_on) idle.swap(g_rt);
+    }
     for (wq3d_queue* q : drop) {
         DeviceGuard guard(q->device);
         delete q;
     }
+    for (QueueRt& rt : idle) {
+        DeviceGuard guard(rt.device);
+        rt.destroy();
+    }
+    if (max_queues == 0) trim_pools();
     return WQ3D_OK;
 }
 
@@ -1599,7 +1739,6 @@ int wq3d_queue_create(const wq3d_ocean* ocean, const wq3d_queue_desc* d, wq3d_qu
     if (reuse) {
         /* the run state of a fresh queue; the device buffers stay */
         old_h = q->h;
-        q->reuse = true;
         q->time = q->ltime = 0.0;
         q->steps = q->lsteps = 0;
         q->carry_refl.clear();
@@ -1651,8 +1790,14 @@ int wq3d_queue_create(const wq3d_ocean* ocean, const wq3d_queue_desc* d, wq3d_qu
         return rc;
     };
     int rc = 0;
-    if (!reuse && cudaStreamCreateWithFlags(&q->stream, cudaStreamNonBlocking) != cudaSuccess)
-        return cleanup(fail(WQ3D_ERR_CUDA, "cudaStreamCreate failed"));
+    const size_t set_bytes = 128 + (((size_t)q->chunk + 1) * sizeof(double) + 63) / 64 * 64;
+    if (!reuse && !rt_take(d->device, q) && (rc = q->make(d->device, q->chunk, 2 * set_bytes))) {
+        const std::string msg = g_err;
+        q->destroy();
+        delete q;
+        g_err = msg;
+        return rc;
+    }
 
     /* host-side inputs */
     const size_t nde = d->num_de, naz = d->num_az, nf = d->num_freq;
@@ -1722,7 +1867,6 @@ int wq3d_queue_create(const wq3d_ocean* ocean, const wq3d_queue_desc* d, wq3d_qu
     std::vector<CpaPatch> patches;
     if (nt) cpa_patches(de, az, nt, &patches);
     h.n_patch = (int)patches.size();
-    patches.resize(nt ? cpa_patch_limit(nde, naz) : 0); /* a reused queue keeps its buffer */
     /* spreading normalisation (spreading_hybrid_gaussian.cc:28-59,
      * spreading_ray.cc:26-45) */
     std::vector<double> norm_de(nde, 0.0), norm_az(n, 0.0), init_area(n, 0.0);
@@ -1750,19 +1894,36 @@ int wq3d_queue_create(const wq3d_ocean* ocean, const wq3d_queue_desc* d, wq3d_qu
         for (auto& v : norm_az) v /= s;
     }
 
-    if ((rc = q->upload(&h.freq, freq)) || (rc = q->upload(&h.alpha, alpha)) ||
-        (rc = q->upload(&h.de, de)) || (rc = q->upload(&h.de_inc, de_inc)) ||
-        (rc = q->upload(&h.az, az)) || (rc = q->upload(&h.az_inc, az_inc)) ||
-        (rc = q->upload(&h.cos_de, cos_de)) || (rc = q->upload(&h.sin_de, sin_de)) ||
-        (rc = q->upload(&h.cos_az, cos_az)) || (rc = q->upload(&h.sin_az, sin_az)) ||
-        (rc = q->upload(&h.tgt[0], tr)) || (rc = q->upload(&h.tgt[1], tt)) ||
-        (rc = q->upload(&h.tgt[2], tp)) || (rc = q->upload(&h.tgt_sin, tsin)) ||
-        (rc = q->upload(&h.tgt_R2, tR2)) || (rc = q->upload(&h.tgt_2R, t2R)) ||
-        (rc = q->upload(&h.tgt_spread2, tspread)) || (rc = q->upload(&h.tgt_c, tc)) ||
-        (rc = q->upload(&h.patches, patches)) || (rc = q->upload(&h.clusters, cpa.clusters)) || (rc = q->upload(&h.cpa_tgt, cpa.tgt)) ||
-        (rc = q->upload(&h.cpa_index, cpa.index)) || (rc = q->upload(&h.de_branch, tbranch)) || (rc = q->upload(&h.norm_de, norm_de)) ||
-        (rc = q->upload(&h.norm_az, norm_az)) || (rc = q->upload(&h.init_area, init_area)))
-        return cleanup(rc);
+    {
+        wq3d_queue::Inputs in;
+        in.add(&h.freq, freq);
+        in.add(&h.alpha, alpha);
+        in.add(&h.de, de);
+        in.add(&h.de_inc, de_inc);
+        in.add(&h.az, az);
+        in.add(&h.az_inc, az_inc);
+        in.add(&h.cos_de, cos_de);
+        in.add(&h.sin_de, sin_de);
+        in.add(&h.cos_az, cos_az);
+        in.add(&h.sin_az, sin_az);
+        in.add(&h.tgt[0], tr);
+        in.add(&h.tgt[1], tt);
+        in.add(&h.tgt[2], tp);
+        in.add(&h.tgt_sin, tsin);
+        in.add(&h.tgt_R2, tR2);
+        in.add(&h.tgt_2R, t2R);
+        in.add(&h.tgt_spread2, tspread);
+        in.add(&h.tgt_c, tc);
+        in.add(&h.de_branch, tbranch);
+        in.add(&h.patches, patches);
+        in.add(&h.clusters, cpa.clusters);
+        in.add(&h.cpa_tgt, cpa.tgt);
+        in.add(&h.cpa_index, cpa.index);
+        in.add(&h.norm_de, norm_de);
+        in.add(&h.norm_az, norm_az);
+        in.add(&h.init_area, init_area);
+        if ((rc = q->upload(in))) return cleanup(rc);
+    }
 
     /* wavefront ring: one allocation carved into 256-byte aligned arrays */
     {
@@ -1827,7 +1988,7 @@ int wq3d_queue_create(const wq3d_ocean* ocean, const wq3d_queue_desc* d, wq3d_qu
         h.cand = cand;
         /* items of the CPA search: a few per patch at most on the measured
          * workloads; k_cpa decides those that find no room */
-        h.cap_item = (uint32_t)std::max<size_t>(4096, std::min<size_t>((size_t)1 << 20, 8 * patches.size()));
+        h.cap_item = (uint32_t)std::max<size_t>(4096, std::min<size_t>((size_t)1 << 20, 2 * n));
         if ((rc = q->alloc(&h.items, h.cap_item))) return cleanup(rc);
         if ((rc = q->alloc(&h.rec, h.cap_rec)) || (rc = q->alloc(&h.rec_inten, (size_t)h.cap_rec * nf)) ||
             (rc = q->alloc(&h.rec_phase, (size_t)h.cap_rec * nf)) || (rc = q->alloc(&h.refl, h.cap_refl)))
@@ -1867,9 +2028,6 @@ int wq3d_queue_create(const wq3d_ocean* ocean, const wq3d_queue_desc* d, wq3d_qu
     h.want_refl = 0;
     {
         /* per result set: base step, counters, chunk times */
-        const size_t set_bytes = 128 + (((size_t)q->chunk + 1) * sizeof(double) + 63) / 64 * 64;
-        if (!reuse && cudaMallocHost(&q->pinned, 2 * set_bytes) != cudaSuccess)
-            return cleanup(fail(WQ3D_ERR_NOMEM, "cudaMallocHost failed"));
         for (int s = 0; s < 2; ++s) {
             char* b = static_cast<char*>(q->pinned) + s * set_bytes;
             q->h_base[s] = reinterpret_cast<int64_t*>(b);
@@ -1879,12 +2037,6 @@ int wq3d_queue_create(const wq3d_ocean* ocean, const wq3d_queue_desc* d, wq3d_qu
     }
     if (cudaMemsetAsync(q->d_counts, 0, 24 * sizeof(uint32_t), q->stream) != cudaSuccess)
         return cleanup(fail(WQ3D_ERR_CUDA, "cudaMemsetAsync failed"));
-    /* The queue's streams do not wait for the default stream, on which the
-     * uploads above were made: the start-up must follow the zeroed counters
-     * (cleared on its own stream) and the last of those copies. */
-    if (cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess)
-        return cleanup(fail(WQ3D_ERR_CUDA, "upload failed"));
-
     /* wave_queue ctor: init_wave, update, init_wavefronts */
     q->gridded = ocean->dev.prof.kind == WQ3D_PROFILE_GRID || ocean->dev.surf.kind == WQ3D_BOUNDARY_GRID ||
                  ocean->dev.bot.kind == WQ3D_BOUNDARY_GRID;
@@ -1893,48 +2045,17 @@ int wq3d_queue_create(const wq3d_ocean* ocean, const wq3d_queue_desc* d, wq3d_qu
     q->k_advance_inline_fn = q->gridded ? gridded::k_advance_inline : analytic::k_advance_inline;
     (q->gridded ? gridded::k_startup : analytic::k_startup)<<<(unsigned)((n + 127) / 128), 128, 0, q->stream>>>(
         h);
-    cudaError_t e = cudaStreamSynchronize(q->stream);
-    if (e == cudaSuccess) e = cudaGetLastError();
-    if (e != cudaSuccess) return cleanup(fail(WQ3D_ERR_CUDA, std::string("start-up kernel: ") + cudaGetErrorString(e)));
     /* spreading_ray.cc:44: sound speed of ray (0,0) on the first front */
-    if (cudaMemcpy(&h.init_sound_speed, h.F[2].c, sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess)
-        return cleanup(fail(WQ3D_ERR_CUDA, "cudaMemcpy failed"));
-    if (!reuse) {
-        if (cudaEventCreate(&q->ev_begin) != cudaSuccess || cudaEventCreate(&q->ev_end) != cudaSuccess)
-            return cleanup(fail(WQ3D_ERR_CUDA, "cudaEventCreate failed"));
-        /* the reflections are the longest chain of a step (one thread per
-         * reflecting ray): their blocks go first when SMs free up */
-        int prio_low = 0, prio_high = 0;
-        if (cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high) != cudaSuccess) prio_high = 0;
-        if (cudaStreamCreateWithPriority(&q->side, cudaStreamNonBlocking, prio_high) != cudaSuccess ||
-            cudaStreamCreateWithFlags(&q->eig, cudaStreamNonBlocking) != cudaSuccess ||
-            cudaStreamCreateWithFlags(&q->adv, cudaStreamNonBlocking) != cudaSuccess ||
-            cudaStreamCreateWithFlags(&q->copy, cudaStreamNonBlocking) != cudaSuccess)
-            return cleanup(fail(WQ3D_ERR_CUDA, "cudaStreamCreate failed"));
-        if (cudaEventCreateWithFlags(&q->eig_end, cudaEventDisableTiming) != cudaSuccess ||
-            cudaEventCreateWithFlags(&q->start_ev, cudaEventDisableTiming) != cudaSuccess)
-            return cleanup(fail(WQ3D_ERR_CUDA, "cudaEventCreate failed"));
-        for (auto& e : q->done_ev)
-            if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
-                return cleanup(fail(WQ3D_ERR_CUDA, "cudaEventCreate failed"));
-        for (auto* v : {&q->fork_ev, &q->join_ev, &q->adv_ev, &q->com_ev, &q->cpa_ev}) {
-            v->resize(q->chunk);
-            for (int k = 0; k < q->chunk; ++k)
-                if (cudaEventCreateWithFlags(&(*v)[k], cudaEventDisableTiming) != cudaSuccess)
-                    return cleanup(fail(WQ3D_ERR_CUDA, "cudaEventCreate failed"));
-        }
-    }
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(q->h_base[0], h.F[2].c, sizeof(double), cudaMemcpyDeviceToHost, q->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(q->stream);
+    if (e != cudaSuccess) return cleanup(fail(WQ3D_ERR_CUDA, std::string("start-up kernel: ") + cudaGetErrorString(e)));
+    std::memcpy(&h.init_sound_speed, q->h_base[0], sizeof(double));
     /* the chunk graphs hold the descriptor by value */
     if (reuse && std::memcmp(&old_h, &h, sizeof(h)) != 0) q->drop_graph();
-    q->reuse = false;
     /* set-up a run would otherwise do on its first chunks: the second
-     * result set and the side-stream graphs of the chunks that reflect
-     * the next chunk's first step (rebuilt later only if callbacks,
-     * thresholds or sensitivities change the descriptor); the graphs of a
-     * run's last full chunk and of the inline schedule are built when
-     * first used */
+     * result set */
     q->ensure_set1();
-    for (int p = 0; p < (q->have_set1 ? 2 : 1); ++p) q->build_graph(p, true, false);
     *out = q;
     return WQ3D_OK;
 }
