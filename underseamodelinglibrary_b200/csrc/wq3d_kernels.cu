@@ -228,6 +228,9 @@ __device__ __forceinline__ void update_main(const QueueDev& q, const FrontPtrs& 
     }
 }
 
+/* a / r.b, by quot() when the time step's powers are in its range */
+__device__ __forceinline__ double div_dt(const QueueDev& q, double a, Recip r) { return q.dt_ok ? quot(a, r) : a / r.b; }
+
 #if !WQ3D_STEP_KERNELS_ONLY
 /* wave_queue::collision_location (wave_queue.cc:982-1057) */
 __device__ void collision_location(const QueueDev& q, const FrontPtrs& V,
@@ -235,22 +238,21 @@ __device__ void collision_location(const QueueDev& q, const FrontPtrs& V,
                                    double tw, double* pos, double* nd,
                                    double* speed) {
     const double dt = q.dt;
-    const double time1 = 2.0 * dt;
-    const double time2 = dt * dt;
+    const Recip time1{2.0 * dt, q.r_2dt}, time2{dt * dt, q.r_dt2};
     const double dtime2 = tw * tw;
-    const double drho = (X.c[i] - V.c[i]) / time1;
-    const double d2rho = (X.c[i] + V.c[i] - 2.0 * C.c[i]) / time2;
+    const double drho = div_dt(q, X.c[i] - V.c[i], time1);
+    const double d2rho = div_dt(q, X.c[i] + V.c[i] - 2.0 * C.c[i], time2);
     *speed = C.c[i] + drho * tw + 0.5 * d2rho * dtime2;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const double v1 = (X.pos[k][i] - V.pos[k][i]) / time1;
-        const double v2 = (X.pos[k][i] + V.pos[k][i] - 2.0 * C.pos[k][i]) / time2;
+        const double v1 = div_dt(q, X.pos[k][i] - V.pos[k][i], time1);
+        const double v2 = div_dt(q, X.pos[k][i] + V.pos[k][i] - 2.0 * C.pos[k][i], time2);
         pos[k] = C.pos[k][i] + v1 * tw + 0.5 * v2 * dtime2;
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const double v1 = (X.nd[k][i] - V.nd[k][i]) / time1;
-        const double v2 = (X.nd[k][i] + V.nd[k][i] - 2.0 * C.nd[k][i]) / time2;
+        const double v1 = div_dt(q, X.nd[k][i] - V.nd[k][i], time1);
+        const double v2 = div_dt(q, X.nd[k][i] + V.nd[k][i] - 2.0 * C.nd[k][i], time2);
         nd[k] = C.nd[k][i] + v1 * tw + 0.5 * v2 * dtime2;
     }
 }
@@ -294,9 +296,6 @@ __device__ __forceinline__ RayC rayc_of(const RayS& y) {
     o.c = y.c;
     return o;
 }
-
-/* a / r.b, by quot() when the time step's powers are in its range */
-__device__ __forceinline__ double div_dt(const QueueDev& q, double a, Recip r) { return q.dt_ok ? quot(a, r) : a / r.b; }
 
 /* wave_queue::collision_location (wave_queue.cc:982-1057) from one ray's
  * prev, curr and next states */
@@ -1917,8 +1916,22 @@ namespace {
  * terms of the beam walks, the per-frequency sums); every value that feeds
  * a rounding-sensitive recurrence (cell distances, the running intensity
  * and its threshold test) is formed in the reference's sequential order,
- * so results equal the one-thread-per-eigenray evaluation. */
-constexpr int EIG_FG = 8; /* frequencies per pass of a walk chunk's Gaussian terms */
+ * so results equal the one-thread-per-eigenray evaluation.
+ *
+ * A step has few candidates, and the next step's commit waits for them, so
+ * what counts is one candidate's latency.  A cell's width is up to four
+ * distances of four sines each, 200 cycles a sine: one pass forms the widths
+ * of the cells on either side of the ray, lanes sharing the sines of their
+ * common ray, where most walks end (three passes of 32 before).  The
+ * recurrences run on every lane from widths and terms in shared memory, two
+ * additions a cell, instead of five shuffles; the terms that the threshold
+ * test needs are those that the lowest frequency adds; and divisions are
+ * branch-free.  Per launch, with the event timing's overhead: 29.7 -> 24.3 us
+ * (Munk workload, one or two candidates a step), 65 -> 46 us (sloped
+ * workload, 907 x 53 rays); 300 -> 315 us with 32 frequencies, whose sums
+ * dominate. */
+constexpr int EIG_FG = 8;    /* frequencies per pass of a walk chunk's Gaussian terms */
+constexpr int EIG_SIDE = 16; /* cells on a side whose widths the first pass forms     */
 
 struct WarpBuild {
     const QueueDev* q;
@@ -1929,11 +1942,38 @@ struct WarpBuild {
     int lane;
     double Ilo, Ihi;         /* running intensity of frequencies lane, lane+32 */
     double (*sg)[EIG_FG + 1]; /* this warp's [cell][frequency] Gaussian terms */
+    double* sw;               /* this warp's cell widths: [32], of the first pass the lower side's */
+    double* su;               /* [16] and the upper side's                    */
+    double u, v;              /* the walk's offset in time and across, in spacings */
+    const FrontPtrs* p2;      /* the front that the time offset leads to      */
 
+    static __device__ __forceinline__ double sine(double x) {
+        double s, c;
+        sin_cos(x, &s, &c);
+        return s;
+    }
+    /* wvector1::distance of two rays whose sines of theta are known */
+    static __device__ __forceinline__ double dist(double r1, double t1, double p1, double s1, double r2, double t2,
+                                                  double p2, double s2) {
+        const double st = sine(0.5 * (t1 - t2));
+        const double sp = sine(0.5 * (p1 - p2));
+        const double dn = 1.0 - 2.0 * (st * st + s1 * s2 * sp * sp);
+        const double dot = r1 * r2 * dn;
+        return sqrt(fabs(r1 * r1 + r2 * r2 - 2.0 * dot));
+    }
     __device__ double fdist(const FrontPtrs& f, int d1, int a1, int d2, int a2) const {
         const int i = d1 * q->naz + a1, j = d2 * q->naz + a2;
-        return sqrt(wdist2(f.pos[0][i], f.pos[1][i], f.pos[2][i], f.pos[0][j],
-                           f.pos[1][j], f.pos[2][j]));
+        const double t1 = f.pos[1][i], t2 = f.pos[1][j];
+        return dist(f.pos[0][i], t1, f.pos[2][i], sine(t1), f.pos[0][j], t2, f.pos[2][j], sine(t2));
+    }
+    /* the same for rays (d, a) and (d + 1, a), where lane "next" has d + 1;
+     * called by a whole warp */
+    __device__ double fdist_de(const FrontPtrs& f, int d, int a, int next) const {
+        const int i = d * q->naz + a, j = min(d + 1, q->nde - 1) * q->naz + a;
+        const double t1 = f.pos[1][i];
+        const double s1 = sine(t1);
+        const double s2 = __shfl_sync(0xffffffffu, s1, next);
+        return dist(f.pos[0][i], t1, f.pos[2][i], s1, f.pos[0][j], f.pos[1][j], f.pos[2][j], s2);
     }
     __device__ double de_inc(int d) const { return q->de_inc[min(max(d, 0), q->nde - 1)]; }
     __device__ double az_inc(int a) const { return q->az_inc[min(max(a, 0), q->naz - 1)]; }
@@ -1941,7 +1981,12 @@ struct WarpBuild {
     /* spreading_hybrid_gaussian.h:148-153 for one frequency */
     __device__ double gauss(double d, double w, double A, int f) const {
         const double bw = spread2[f] + 2.0 * 2.0 * w * w;
-        return exp((-0.5 * d * d) / bw) / sqrt(bw) * A;
+        const double e = -0.5 * d * d, s = sqrt(bw);
+        if (divisor_ok(bw) && divisor_ok(s) && dividend_ok(e)) {
+            const double g = exp(quot(e, recip(bw)));
+            return (dividend_ok(g) ? quot(g, recip(s)) : g / s) * A;
+        }
+        return exp(e / bw) / s * A;
     }
     /* running intensity += gaussian, frequencies spread over the lanes */
     __device__ void acc(double d, double w, double A, bool first) {
@@ -1957,204 +2002,182 @@ struct WarpBuild {
     }
     __device__ double I0() const { return __shfl_sync(0xffffffffu, Ilo, 0); }
 
-    /* The lowest frequency's running intensity over cells 0..ncell-1 (lane
-     * k holds cell k's term g0), added in cell order, and the reference's
-     * threshold test after each cell (new / old < 1.002305238).  Returns
-     * the first cell that passes it, or -1.  The sums are sequential; the
-     * divisions of the tests are not, so they run on all lanes at once. */
-    __device__ int threshold_cell(int ncell, double g0) const {
-        double i0 = I0();
-        double my_new = 1.0, my_old = 1.0;
-        for (int k = 0; k < ncell; ++k) {
-            const double old = i0;
-            i0 += __shfl_sync(0xffffffffu, g0, k);
-            if (lane == k) {
-                my_new = i0;
-                my_old = old;
-            }
-        }
-        const unsigned hit = __ballot_sync(0xffffffffu, lane < ncell && my_new / my_old < 1.002305238);
-        return hit ? __ffs(hit) - 1 : -1;
-    }
-
-    /* acc() of cells 0..ncell-1 in cell order, for every frequency: lane k
-     * computes cell k's Gaussian terms (EIG_FG frequencies per pass), then
-     * the lane that owns a frequency adds them up in cell order */
-    __device__ void acc_cells(int ncell, double cd, double cw, double nm) {
+    /* Cells 0..nend-1 of a walk, whose distance, width and normalisation
+     * lane k holds for cell k: the reference's threshold test on the lowest
+     * frequency's running intensity after each cell (new / old <
+     * 1.002305238), then every frequency's sum over the cells up to the first
+     * that passes, or all; both in cell order.  The sums are sequential; the
+     * divisions of the tests are not, so they run on all lanes at once.
+     * Returns the first cell that passes the test, or -1. */
+    __device__ int add_cells(int nend, double cd, double cw, double nm) {
         const int nf = q->nf;
+        int last = nend - 1, hit_cell = -1;
         for (int f0 = 0; f0 < nf; f0 += EIG_FG) {
             const int nfg = min(EIG_FG, nf - f0);
-            if (lane < ncell)
+            if (lane <= last)
                 for (int j = 0; j < nfg; ++j) sg[lane][j] = gauss(cd, cw, nm, f0 + j);
             __syncwarp();
+            if (f0 == 0) {
+                double i0 = I0(), my_new = 1.0, my_old = 1.0;
+#pragma unroll 4
+                for (int k = 0; k < nend; ++k) {
+                    const double old = i0;
+                    i0 += sg[k][0];
+                    if (lane == k) {
+                        my_new = i0;
+                        my_old = old;
+                    }
+                }
+                const unsigned hit = __ballot_sync(0xffffffffu, lane < nend && my_new / my_old < 1.002305238);
+                if (hit) last = hit_cell = __ffs(hit) - 1;
+            }
             if (lane >= f0 && lane < f0 + nfg) {
                 double I = Ilo;
-                for (int k = 0; k < ncell; ++k) I = I + sg[k][lane - f0];
+#pragma unroll 4
+                for (int k = 0; k <= last; ++k) I = I + sg[k][lane - f0];
                 Ilo = I;
             }
             if (lane + 32 >= f0 && lane + 32 < f0 + nfg) {
                 double I = Ihi;
-                for (int k = 0; k < ncell; ++k) I = I + sg[k][lane + 32 - f0];
+#pragma unroll 4
+                for (int k = 0; k <= last; ++k) I = I + sg[k][lane + 32 - f0];
                 Ihi = I;
             }
             __syncwarp();
         }
+        return hit_cell;
     }
 
-    /* spreading_hybrid_gaussian.cc:430-495 */
-    __device__ double width_de(int d, int a, const double* offset) const {
-        const double u = fabs(offset[0]) / q->dt;
-        const double v = fabs(offset[2]) / az_inc(a);
-        const int max_az = q->naz - 1;
-        const int az_wrap = (a + 1 >= max_az) ? 0 : a + 1;
-        const FrontPtrs& C = *pC;
-        double L1 = fdist(C, d, a, d + 1, a), L2, length1, length2;
-        if (v < 1e-10) {
-            length1 = L1;
-        } else {
-            L2 = fdist(C, d, az_wrap, d + 1, az_wrap);
-            length1 = (1.0 - v) * L1 + v * L2;
-        }
+    /* u, v and p2 of a walk: |offset in time| over the step, |offset across|
+     * over its spacing */
+    __device__ void set_offsets(double dtime, double across, double spacing) {
+        u = fabs(dtime) / q->dt;
+        v = fabs(across) / spacing;
+        p2 = (dtime < 0.0) ? pV : pX;
+    }
+
+    /* the blend of the four distances (spreading_hybrid_gaussian.cc:430-571) */
+    template <class F>
+    __device__ double width(bool cross, F column) const {
+        double L1 = column(*pC, 0);
+        const double length1 = cross ? (1.0 - v) * L1 + v * column(*pC, 1) : L1;
         if (u < 1e-10) return 0.5 * length1;
-        const FrontPtrs& p2 = (offset[0] < 0.0) ? *pV : *pX;
-        L1 = fdist(p2, d, a, d + 1, a);
-        if (v < 1e-10) {
-            length2 = L1;
-        } else {
-            L2 = fdist(p2, d, az_wrap + 1, d + 1, az_wrap + 1);
-            length2 = (1.0 - v) * L1 + v * L2;
-        }
+        L1 = column(*p2, 0);
+        const double length2 = cross ? (1.0 - v) * L1 + v * column(*p2, 2) : L1;
         return 0.5 * ((1.0 - u) * length1 + u * length2);
     }
 
+    /* spreading_hybrid_gaussian.cc:430-495; "next": the lane with ray d + 1
+     * (a whole warp then calls it), or -1 */
+    __device__ double width_de(int d, int a, int next) const {
+        const int max_az = q->naz - 1;
+        const int az_wrap = (a + 1 >= max_az) ? 0 : a + 1;
+        return width(!(v < 1e-10), [&](const FrontPtrs& f, int side) {
+            const int col = side == 0 ? a : side == 1 ? az_wrap : az_wrap + 1;
+            return next < 0 ? fdist(f, d, col, d + 1, col) : fdist_de(f, d, col, next);
+        });
+    }
+
     /* spreading_hybrid_gaussian.cc:500-571 */
-    __device__ double width_az(int d, int a, const double* offset) const {
-        const double u = fabs(offset[0]) / q->dt;
-        const double v = fabs(offset[1]) / de_inc(d);
+    __device__ double width_az(int d, int a) const {
         const int max_az = q->naz - 1;
         const int max_de = q->nde - 1;
         const int de_upper = (d + 1 >= max_de) ? max_de - 2 : d;
         const int az_wrap = (a + 1 > max_az) ? 0 : a + 1;
-        const FrontPtrs& C = *pC;
-        double L1 = fdist(C, d, a, d, az_wrap), L2, length1, length2;
-        if (v < 1e-10 || fabs(v - 1.0) < 1e-10) {
-            length1 = L1;
-        } else {
-            L2 = fdist(C, de_upper + 1, a, de_upper + 1, az_wrap);
-            length1 = (1.0 - v) * L1 + v * L2;
-        }
-        if (u < 1e-10) return 0.5 * length1;
-        const FrontPtrs& p2 = (offset[0] < 0.0) ? *pV : *pX;
-        L1 = fdist(p2, d, a, d, az_wrap);
-        if (v < 1e-10 || fabs(v - 1.0) < 1e-10) {
-            length2 = L1;
-        } else {
-            L2 = fdist(p2, de_upper + 1, a, de_upper + 1, az_wrap);
-            length2 = (1.0 - v) * L1 + v * L2;
-        }
-        return 0.5 * ((1.0 - u) * length1 + u * length2);
+        return width(!(v < 1e-10 || fabs(v - 1.0) < 1e-10), [&](const FrontPtrs& f, int side) {
+            const int row = side == 0 ? d : de_upper + 1;
+            return fdist(f, row, a, row, az_wrap);
+        });
     }
 
-    /* Processes up to 32 prepared cells of one walk.  Lane k holds cell k's
-     * width (w_k), whether the cell is a virtual ray (virt_k) and the two
-     * normalisation candidates.  sign = +1 for a walk away from the lower
-     * side (cell distances grow), -1 otherwise.  Returns true when the walk
-     * stops inside these cells. */
-    __device__ bool run_cells(int ncell, double w_k, bool virt_k, double norm_k,
-                              double norm_virt_k, double sign, double& cell_dist,
-                              double& cell_width) {
-        double my_cd = 0.0, my_cw = 0.0, my_nm = 0.0;
-        int nend = ncell;
-        bool stop = false;
-        for (int k = 0; k < ncell; ++k) {
-            const bool v = __shfl_sync(0xffffffffu, virt_k, k);
-            const double wk = __shfl_sync(0xffffffffu, w_k, k);
-            const double nk = __shfl_sync(0xffffffffu, v ? norm_virt_k : norm_k, k);
-            if (sign > 0.0) {
-                cell_dist += cell_width;
-                if (v) {
-                    cell_dist += cell_width;
-                } else {
-                    cell_width = wk;
-                    cell_dist += cell_width;
-                }
-            } else {
-                cell_dist -= cell_width;
-                if (v) {
-                    cell_dist -= cell_width;
-                } else {
-                    cell_width = wk;
-                    cell_dist -= cell_width;
-                }
-            }
+    /* Processes up to 32 cells of one walk, whose widths are w[0..ncell-1] in
+     * shared memory.  Lane k holds whether cell k is a virtual ray (virt_k,
+     * where the walk ends) and its two normalisation candidates.  sign = +1
+     * for a walk away from the lower side, -1 for the upper.  Returns true
+     * when the walk ends; *stop: the cell it passed the threshold on, if so. */
+    __device__ bool run_cells(int ncell, const double* w, bool virt_k, double norm_k, double norm_virt_k,
+                              double sign, double& cell_dist, double& cell_width, int* stop) {
+        const unsigned virt = __ballot_sync(0xffffffffu, lane < ncell && virt_k);
+        const int nend = virt ? __ffs(virt) : ncell; /* cells used; the last may be virtual */
+        double my_cd = 0.0, my_cw = 0.0;
+        double cd = cell_dist, cw = cell_width;
+#pragma unroll 4
+        for (int k = 0; k < nend; ++k) {
+            const double wk = w[k];
+            const bool keep = virt && k == nend - 1; /* a virtual ray keeps the width */
+            cd = sign > 0.0 ? cd + cw : cd - cw;
+            if (!keep) cw = wk;
+            cd = sign > 0.0 ? cd + cw : cd - cw;
             if (lane == k) {
-                my_cd = cell_dist;
-                my_cw = cell_width;
-                my_nm = nk;
-            }
-            if (v) {
-                nend = k + 1;
-                stop = true;
-                break;
+                my_cd = cd;
+                my_cw = cw;
             }
         }
-        /* threshold scan on the lowest frequency, in order */
-        const double g0 = (lane < nend) ? gauss(my_cd, my_cw, my_nm, 0) : 0.0;
-        int kstar = threshold_cell(nend, g0);
-        if (kstar >= 0) {
-            stop = true;
-        } else {
-            kstar = nend - 1;
-        }
-        /* accumulate every frequency over cells 0..kstar, in order */
-        acc_cells(kstar + 1, my_cd, my_cw, my_nm);
-        return stop;
+        cell_dist = cd;
+        cell_width = cw;
+        const int hit = add_cells(nend, my_cd, my_cw, virt && lane == nend - 1 ? norm_virt_k : norm_k);
+        if (hit >= 0) *stop = hit;
+        return hit >= 0 || virt != 0;
     }
 
     /* spreading_hybrid_gaussian.cc:124-258 */
     __device__ void intensity_de(int de0, int a, const double* offset, const double* distance) {
         const QueueDev& Q = *q;
         const FrontPtrs& C = *pC;
-        double wl = 0.0, wc = 0.0;
-        if (lane == 0) wc = width_de(de0, a, offset);
-        if (lane == 1) wl = width_de(de0 - 1, a, offset);
-        wc = __shfl_sync(0xffffffffu, wc, 0);
-        wl = __shfl_sync(0xffffffffu, wl, 1);
+        set_offsets(offset[0], offset[2], az_inc(a));
+        /* lanes 0-15: cells de0-1, de0-2, ...; lanes 16-30: cells de0, de0+1, ... */
+        {
+            const bool lower = lane < EIG_SIDE;
+            const int d = lower ? max(de0 - 1 - lane, 0) : min(de0 + lane - EIG_SIDE, Q.nde - 1);
+            const double w = width_de(d, a, lower ? (lane == 0 ? EIG_SIDE : lane - 1) : min(lane + 1, 31));
+            if (lower)
+                sw[lane] = w;
+            else
+                su[lane - EIG_SIDE] = w;
+        }
+        __syncwarp();
+        const double wl = sw[0], wc = su[0];
         const double L = distance[1];
         acc(L - wc, wc, Q.norm_de[de0], true);
         acc(L + wl, wl, Q.norm_de[de0 - 1], false);
         if (I0() < 1e-10) return;
-        /* lower D/E cells: de0-2 down to 0 */
+        int stop;
+        /* lower D/E cells: de0-2 down to 0; "at" 1 while the first pass's
+         * widths serve */
         double cell_width = wl, cell_dist = L + wl;
-        for (int d0 = de0 - 2; d0 >= 0; d0 -= 32) {
+        for (int d0 = de0 - 2, at = 1; d0 >= 0; at = 0) {
             const int d = d0 - lane;
-            const int ncell = min(32, d0 + 1);
+            const int ncell = min(at ? EIG_SIDE - 1 : 32, d0 + 1);
             bool virt = false;
-            double w = 0.0, nm = 0.0, nmv = 0.0;
+            double nm = 0.0, nmv = 0.0;
             if (lane < ncell) {
                 virt = C.on_edge[(d + 1) * Q.naz + a] && C.on_edge[d * Q.naz + a];
-                if (!virt) w = width_de(d, a, offset);
                 nm = Q.norm_de[d];
                 nmv = Q.norm_de[d + 1];
+                if (!at && !virt) sw[lane] = width_de(d, a, -1);
             }
-            if (run_cells(ncell, w, virt, nm, nmv, 1.0, cell_dist, cell_width)) break;
+            __syncwarp();
+            if (run_cells(ncell, sw + at, virt, nm, nmv, 1.0, cell_dist, cell_width, &stop)) break;
+            d0 -= ncell;
         }
         /* upper D/E cells: de0+1 up to num_de-2 */
         cell_width = wc;
         cell_dist = L - wc;
         const int size = Q.nde - 1;
-        for (int d0 = de0 + 1; d0 < size; d0 += 32) {
+        for (int d0 = de0 + 1, at = 1; d0 < size; at = 0) {
             const int d = d0 + lane;
-            const int ncell = min(32, size - d0);
+            const int ncell = min(at ? EIG_SIDE - 2 : 32, size - d0);
             bool virt = false;
-            double w = 0.0, nm = 0.0, nmv = 0.0;
+            double nm = 0.0, nmv = 0.0;
             if (lane < ncell) {
                 virt = C.on_edge[(d + 1) * Q.naz + a] && C.on_edge[d * Q.naz + a];
-                if (!virt) w = width_de(d, a, offset);
                 nm = Q.norm_de[d];
                 nmv = Q.norm_de[d - 1];
+                if (!at && !virt) sw[lane] = width_de(d, a, -1);
             }
-            if (run_cells(ncell, w, virt, nm, nmv, -1.0, cell_dist, cell_width)) break;
+            __syncwarp();
+            if (run_cells(ncell, at ? su + 1 : sw, virt, nm, nmv, -1.0, cell_dist, cell_width, &stop)) break;
+            d0 += ncell;
         }
     }
 
@@ -2170,21 +2193,26 @@ struct WarpBuild {
         const int az_upper = Q.az_boundary ? az0 : max_az - 1;
         auto norm = [&](int aa) { return (d >= max_de) ? Q.norm_az[1 * Q.naz + aa] : Q.norm_az[d * Q.naz + aa]; };
         const int a1 = (az0 < 1) ? max_az - 1 : az0 - 1;
-        double wc = 0.0, wl = 0.0;
-        if (lane == 0) wc = width_az(d, az0, offset);
-        if (lane == 1) wl = width_az(d, a1, offset);
-        wc = __shfl_sync(0xffffffffu, wc, 0);
-        wl = __shfl_sync(0xffffffffu, wl, 1);
+        const int start = (a1 < 1) ? max_az - 1 : a1 - 1;
+        set_offsets(offset[0], offset[1], de_inc(d));
+        /* lanes 0-15: cells a1, then start, start-1, ... (cyclic); lanes
+         * 16-31: cells az0, az0+1, ... (cyclic) */
+        if (lane < EIG_SIDE)
+            sw[lane] = width_az(d, lane == 0 ? a1 : (((start - (lane - 1)) % max_az) + max_az) % max_az);
+        else
+            su[lane - EIG_SIDE] = width_az(d, lane == EIG_SIDE ? az0 : (az0 + lane - EIG_SIDE) % max_az);
+        __syncwarp();
+        const double wl = sw[0], wc = su[0];
         const double L = distance[2];
         acc(L - wc, wc, norm(az0), true);
         acc(L + wl, wl, norm(a1), false);
         if (I0() < 1e-10) return;
         /* lower walk: a1-1, a1-2, ... (cyclic) until az_lower */
-        const int start = (a1 < 1) ? max_az - 1 : a1 - 1;
         double cell_width = wl, cell_dist = L + wl;
         int marked = -1; /* index (in walk order) of the last cell marked */
         bool done = false;
-        for (int k0 = 0; !done && k0 < max_az; k0 += 32) {
+        for (int k0 = 0, at = 1; !done && k0 < max_az; at = 0) {
+            const int len = at ? EIG_SIDE - 1 : 32;
             const int k = k0 + lane;
             int a = start - k;
             a = ((a % max_az) + max_az) % max_az;
@@ -2197,18 +2225,17 @@ struct WarpBuild {
             } else if (C.on_edge[d * Q.naz + a]) {
                 kind = 2;
             }
-            const unsigned stopmask = __ballot_sync(0xffffffffu, kind != 0);
-            int first = 32, fk = 0;
+            const unsigned stopmask = __ballot_sync(0xffffffffu, kind != 0 && lane < len);
+            int ncell = len, fk = 0;
             if (stopmask) {
-                first = __ffs(stopmask) - 1;
-                fk = __shfl_sync(0xffffffffu, kind, first);
+                ncell = __ffs(stopmask) - 1;
+                fk = __shfl_sync(0xffffffffu, kind, ncell);
             }
-            const int ncell = first;
-            double w = 0.0;
-            if (lane < ncell) w = width_az(d, a, offset);
+            if (!at && lane < ncell) sw[lane] = width_az(d, a);
             const double nm = (lane < ncell) ? norm(a) : 0.0;
+            __syncwarp();
             int kst = -1;
-            const bool brk = (ncell > 0) && run_cells_az(ncell, w, nm, 1.0, cell_dist, cell_width, kst);
+            const bool brk = (ncell > 0) && run_cells(ncell, sw + at, false, nm, nm, 1.0, cell_dist, cell_width, &kst);
             if (brk) {
                 marked = k0 + kst; /* the threshold stop happens on a marked cell */
                 done = true;
@@ -2216,15 +2243,17 @@ struct WarpBuild {
                 if (ncell > 0) marked = k0 + ncell - 1;
                 if (stopmask) {
                     done = true;
-                    if (fk == 2) marked = k0 + first; /* on_edge cells are marked, not used */
+                    if (fk == 2) marked = k0 + ncell; /* on_edge cells are marked, not used */
                 }
             }
+            k0 += len;
         }
         /* upper walk: az0+1, az0+2, ... (cyclic) until az_upper */
         cell_width = wc;
         cell_dist = L - wc;
         done = false;
-        for (int k0 = 0; !done && k0 < max_az; k0 += 32) {
+        for (int k0 = 0, at = 1; !done && k0 < max_az; at = 0) {
+            const int len = at ? EIG_SIDE - 1 : 32;
             const int k = k0 + lane;
             const int a = (az0 + 1 + k) % max_az;
             int kind = 0;
@@ -2238,50 +2267,20 @@ struct WarpBuild {
             } else if (C.on_edge[d * Q.naz + a]) {
                 kind = 1;
             }
-            const unsigned stopmask = __ballot_sync(0xffffffffu, kind != 0);
-            int ncell = 32;
+            const unsigned stopmask = __ballot_sync(0xffffffffu, kind != 0 && lane < len);
+            int ncell = len;
             if (stopmask) {
                 ncell = __ffs(stopmask) - 1;
                 done = true;
             }
-            double w = 0.0;
-            if (lane < ncell) w = width_az(d, a, offset);
+            if (!at && lane < ncell) sw[lane] = width_az(d, a);
             const double nm = (lane < ncell) ? norm(a) : 0.0;
+            __syncwarp();
             int kst = -1;
-            if (ncell > 0 && run_cells_az(ncell, w, nm, -1.0, cell_dist, cell_width, kst)) done = true;
+            if (ncell > 0 && run_cells(ncell, at ? su + 1 : sw, false, nm, nm, -1.0, cell_dist, cell_width, &kst))
+                done = true;
+            k0 += len;
         }
-    }
-
-    /* AZ walks have no virtual rays; a threshold stop marks the cell it
-     * happened on (for the upper walk's duplicate test) */
-    __device__ bool run_cells_az(int ncell, double w_k, double norm_k, double sign,
-                                 double& cell_dist, double& cell_width, int& kstop) {
-        double my_cd = 0.0, my_cw = 0.0, my_nm = 0.0;
-        for (int k = 0; k < ncell; ++k) {
-            const double wk = __shfl_sync(0xffffffffu, w_k, k);
-            const double nk = __shfl_sync(0xffffffffu, norm_k, k);
-            if (sign > 0.0) {
-                cell_dist += cell_width;
-                cell_width = wk;
-                cell_dist += cell_width;
-            } else {
-                cell_dist -= cell_width;
-                cell_width = wk;
-                cell_dist -= cell_width;
-            }
-            if (lane == k) {
-                my_cd = cell_dist;
-                my_cw = cell_width;
-                my_nm = nk;
-            }
-        }
-        const double g0 = (lane < ncell) ? gauss(my_cd, my_cw, my_nm, 0) : 0.0;
-        int kstar = threshold_cell(ncell, g0);
-        const bool stop = kstar >= 0;
-        if (!stop) kstar = ncell - 1;
-        acc_cells(kstar + 1, my_cd, my_cw, my_nm);
-        if (stop) kstop = kstar;
-        return stop;
     }
 
     /* wvector1::area on four points (types/wvector1.cc) */
@@ -2297,32 +2296,67 @@ struct WarpBuild {
     }
 };
 
-__device__ __forceinline__ void make_taylor_coeff(const double v[3][3][3], const double* delta,
-                                                  double& center, double* g, double h[3][3]) {
-    const double d0 = 2.0 * delta[0];
-    const double d1 = 2.0 * delta[1];
-    const double d2 = 2.0 * delta[2];
+/* the spacings that a candidate's Taylor fits divide by, and whether quot()
+ * may divide by all of them; the dividends are differences of distance2 (m^2)
+ * or of degrees, and quotients of those */
+struct TaylorDiv {
+    Recip d[3];   /* delta             */
+    Recip two[3]; /* 2 delta           */
+    Recip sq[3];  /* delta^2           */
+    bool ok;
+    __device__ explicit TaylorDiv(const double* delta) : ok(true) {
+        for (int k = 0; k < 3; ++k) {
+            d[k] = recip(delta[k]);
+            two[k] = recip(2.0 * delta[k]);
+            sq[k] = recip(delta[k] * delta[k]);
+            ok = ok && divisor_ok(delta[k]) && divisor_ok(2.0 * delta[k]) && divisor_ok(delta[k] * delta[k]);
+        }
+    }
+};
+
+template <bool FAST>
+__device__ __forceinline__ double divide(double a, Recip r) {
+    return FAST ? quot(a, r) : a / r.b;
+}
+
+template <bool FAST>
+__device__ __forceinline__ void taylor_coeff(const double v[3][3][3], const TaylorDiv& D, double& center, double* g,
+                                             double h[3][3]) {
     center = v[1][1][1];
-    for (int r = 0; r < 3; ++r)
-        for (int c = 0; c < 3; ++c) h[r][c] = 0.0;
-    h[0][0] = (v[2][1][1] + v[0][1][1] - 2.0 * center) / (delta[0] * delta[0]);
-    h[1][1] = (v[1][2][1] + v[1][0][1] - 2.0 * center) / (delta[1] * delta[1]);
-    h[2][2] = (v[1][1][2] + v[1][1][0] - 2.0 * center) / (delta[2] * delta[2]);
-    g[0] = (v[2][0][1] - v[0][0][1]) / d0;
-    g[2] = (v[2][2][1] - v[0][2][1]) / d0;
-    h[0][1] = (g[2] - g[0]) / d1;
+    h[0][0] = divide<FAST>(v[2][1][1] + v[0][1][1] - 2.0 * center, D.sq[0]);
+    h[1][1] = divide<FAST>(v[1][2][1] + v[1][0][1] - 2.0 * center, D.sq[1]);
+    h[2][2] = divide<FAST>(v[1][1][2] + v[1][1][0] - 2.0 * center, D.sq[2]);
+    g[0] = divide<FAST>(v[2][0][1] - v[0][0][1], D.two[0]);
+    g[2] = divide<FAST>(v[2][2][1] - v[0][2][1], D.two[0]);
+    h[0][1] = divide<FAST>(g[2] - g[0], D.two[1]);
     h[1][0] = h[0][1];
-    g[0] = (v[2][1][0] - v[0][1][0]) / d0;
-    g[2] = (v[2][1][2] - v[0][1][2]) / d0;
-    h[0][2] = (g[2] - g[0]) / d2;
+    g[0] = divide<FAST>(v[2][1][0] - v[0][1][0], D.two[0]);
+    g[2] = divide<FAST>(v[2][1][2] - v[0][1][2], D.two[0]);
+    h[0][2] = divide<FAST>(g[2] - g[0], D.two[2]);
     h[2][0] = h[0][2];
-    g[0] = (v[1][2][0] - v[1][0][0]) / d1;
-    g[2] = (v[1][2][2] - v[1][0][2]) / d1;
-    h[1][2] = (g[2] - g[0]) / d2;
+    g[0] = divide<FAST>(v[1][2][0] - v[1][0][0], D.two[1]);
+    g[2] = divide<FAST>(v[1][2][2] - v[1][0][2], D.two[1]);
+    h[1][2] = divide<FAST>(g[2] - g[0], D.two[2]);
     h[2][1] = h[1][2];
-    g[0] = (v[2][1][1] - v[0][1][1]) / d0;
-    g[1] = (v[1][2][1] - v[1][0][1]) / d1;
-    g[2] = (v[1][1][2] - v[1][1][0]) / d2;
+    g[0] = divide<FAST>(v[2][1][1] - v[0][1][1], D.two[0]);
+    g[1] = divide<FAST>(v[1][2][1] - v[1][0][1], D.two[1]);
+    g[2] = divide<FAST>(v[1][1][2] - v[1][1][0], D.two[2]);
+}
+
+__device__ __forceinline__ void make_taylor_coeff(const double v[3][3][3], const TaylorDiv& D, double& center,
+                                                  double* g, double h[3][3]) {
+    if (D.ok)
+        taylor_coeff<true>(v, D, center, g, h);
+    else
+        taylor_coeff<false>(v, D, center, g, h);
+}
+
+/* m /= x */
+__device__ __forceinline__ void divide_all(double m[3][3], double x) {
+    const Recip r = recip(x);
+    const bool ok = divisor_ok(x);
+    for (int i = 0; i < 3; ++i)
+        for (int j = 0; j < 3; ++j) m[i][j] = ok ? quot(m[i][j], r) : m[i][j] / x;
 }
 
 __device__ __forceinline__ double dot3(const double* a, const double* b) {
@@ -2353,7 +2387,7 @@ __device__ __forceinline__ double norm2(const double* g) {
  * warp: lanes 0-8 test the 3x3 neighbours' stability at once. */
 __device__ void compute_offsets(const QueueDev& q, const FrontPtrs& V, const FrontPtrs& C,
                                 const FrontPtrs& X, int t, int de0, int az0,
-                                const double cube[3][3][3], const double* delta,
+                                const double cube[3][3][3], const double* delta, const TaylorDiv& D,
                                 double* offset, double* distance) {
     const int ic = de0 * q.naz + az0;
     bool bad = false;
@@ -2370,16 +2404,21 @@ __device__ void compute_offsets(const QueueDev& q, const FrontPtrs& V, const Fro
     }
     bool unstable = __any_sync(0xffffffffu, bad);
     double center, g[3], h[3][3], inv[3][3];
-    make_taylor_coeff(cube, delta, center, g, h);
+    make_taylor_coeff(cube, D, center, g, h);
     /* kept: hessian(2,1)*hessian(2,0) in the last cofactor (wave_queue.cc:762-763) */
     double determinant = fmax(1e-6, h[0][0] * (h[1][1] * h[2][2] - h[1][2] * h[2][1]) +
                                         h[0][1] * (h[1][2] * h[2][0] - h[1][0] * h[2][2]) +
                                         h[0][2] * (h[1][0] * h[2][1] - h[2][1] * h[2][0]));
     unstable = unstable || determinant < norm2(g);
+    const double hh[3] = {fmax(1e-10, h[0][0]), fmax(1e-10, h[1][1]), fmax(1e-10, h[2][2])};
+    const bool fast = D.ok && divisor_ok(hh[0]) && divisor_ok(hh[1]) && divisor_ok(hh[2]);
+    double ratio[3];
     for (int k = 0; k < 3; ++k) {
-        const double hh = fmax(1e-10, h[k][k]);
-        offset[k] = -g[k] / hh;
-        if (fabs(offset[k] / delta[k]) > 0.5) {
+        offset[k] = fast ? quot(-g[k], recip(hh[k])) : -g[k] / hh[k];
+        ratio[k] = fast ? quot(offset[k], D.d[k]) : offset[k] / delta[k];
+    }
+    for (int k = 0; k < 3; ++k) {
+        if (fabs(ratio[k]) > 0.5) {
             unstable = true;
             offset[k] = (offset[k] < 0.0) ? -(0.5 * delta[k]) : 0.5 * delta[k];
         }
@@ -2394,8 +2433,7 @@ __device__ void compute_offsets(const QueueDev& q, const FrontPtrs& V, const Fro
         inv[0][2] = inv[2][0];
         inv[1][2] = inv[2][1];
         inv[2][2] = h[0][0] * h[1][1] - h[0][1] * h[1][0];
-        for (int r = 0; r < 3; ++r)
-            for (int c = 0; c < 3; ++c) inv[r][c] /= determinant;
+        divide_all(inv, determinant);
         const double ng[3] = {-g[0], -g[1], -g[2]};
         matvec(inv, ng, offset);
         unstable = unstable || fabs(offset[1]) >= 0.5 * fabs(delta[1]);
@@ -2411,8 +2449,7 @@ __device__ void compute_offsets(const QueueDev& q, const FrontPtrs& V, const Fro
             inv[1][1] = 1.0;
             inv[2][0] = -h[2][0];
             inv[2][2] = h[0][0];
-            for (int r = 0; r < 3; ++r)
-                for (int c = 0; c < 3; ++c) inv[r][c] /= determinant;
+            divide_all(inv, determinant);
             const double ng[3] = {-g[0], -g[1], -g[2]};
             matvec(inv, ng, offset);
             offset[1] = save_offset;
@@ -2469,6 +2506,7 @@ __global__ void __launch_bounds__(32 * EIG_WARPS) k_eigenray(__grid_constant__ c
     __shared__ double s_ang[EIG_WARPS][2][27];
     __shared__ double s_g[EIG_WARPS][32][EIG_FG + 1];
     __shared__ double s_az[EIG_WARPS / 2][64];
+    __shared__ double s_w[EIG_WARPS][32 + EIG_SIDE];
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     /* a warp pair per candidate: with hybrid Gaussian spreading the even
@@ -2487,6 +2525,8 @@ __global__ void __launch_bounds__(32 * EIG_WARPS) k_eigenray(__grid_constant__ c
     B.pX = &q.F[ring_slot(s + 3)];
     B.lane = lane;
     B.sg = s_g[warp];
+    B.sw = s_w[warp];
+    B.su = s_w[warp] + 32;
     const FrontPtrs& V = *B.pV;
     const FrontPtrs& C = *B.pC;
     const FrontPtrs& X = *B.pX;
@@ -2518,7 +2558,8 @@ __global__ void __launch_bounds__(32 * EIG_WARPS) k_eigenray(__grid_constant__ c
         __syncwarp();
         double delta[3] = {q.dt, q.de_inc[de0], q.az_inc[az0]};
         double offset[3], distance[3];
-        compute_offsets(q, V, C, X, t, de0, az0, cube, delta, offset, distance);
+        const TaylorDiv D(delta);
+        compute_offsets(q, V, C, X, t, de0, az0, cube, delta, D, offset, distance);
 
         /* spreading: lane f holds frequency f (and f + 32) */
         double si_lo = 0.0, si_hi = 0.0;
@@ -2614,7 +2655,7 @@ __global__ void __launch_bounds__(32 * EIG_WARPS) k_eigenray(__grid_constant__ c
         double tang[2];
         for (int which = 0; which < 2; ++which) {
             double center, g[3], h[3][3], hv[3];
-            make_taylor_coeff(reinterpret_cast<double (*)[3][3]>(s_ang[warp][which]), delta, center, g, h);
+            make_taylor_coeff(reinterpret_cast<double (*)[3][3]>(s_ang[warp][which]), D, center, g, h);
             matvec(h, offset, hv);
             tang[which] = center + dot3(g, offset) + 0.5 * dot3(offset, hv);
         }
