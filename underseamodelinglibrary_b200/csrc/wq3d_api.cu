@@ -178,19 +178,7 @@ cudaError_t device_pool(int device, cudaMemPool_t* out) {
     return cudaSuccess;
 }
 
-/* bytes that the device's pool holds and no queue uses */
-size_t pool_idle_bytes(int device) {
-    cudaMemPool_t pool;
-    uint64_t held = 0, used = 0;
-    if (device_pool(device, &pool) != cudaSuccess ||
-        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
-        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    return held > used ? (size_t)(held - used) : 0;
-}
-
+/* gives back what the pools hold and no queue uses */
 void trim_pools() {
     std::lock_guard<std::mutex> lock(g_pool_mu);
     for (auto& pool : g_pool)
@@ -198,6 +186,10 @@ void trim_pools() {
 }
 
 }  // namespace
+
+/* when memory is short: gives back the destroyed queues kept for reuse and
+ * what the pools hold idle */
+extern "C" void wq3d_internal_release_idle(void);
 
 struct wq3d_ocean {
     OceanDev dev;   /* device pointers, passed to kernels        */
@@ -291,25 +283,39 @@ int make_grid(wq3d_ocean* o, const wq3d_grid_desc& d, int max_dims, GridDev* hg,
     }
     if (!ok) hg->unrolled = GRID_GENERAL;
     *dg = *hg;
-    auto up = [&](const double* src, size_t n, const double** out) -> int {
-        void* p = nullptr;
-        WQ_CK(cudaMalloc(&p, n * sizeof(double)));
-        o->dmem.push_back(p);
-        WQ_CK(cudaMemcpy(p, src, n * sizeof(double), cudaMemcpyHostToDevice));
-        *out = static_cast<const double*>(p);
-        return WQ3D_OK;
+    /* one allocation, its tables gathered and sent as one copy (a copy and an
+     * allocation for each took 0.1 ms apiece), then the data */
+    std::vector<double> tables;
+    std::vector<std::pair<const double**, size_t>> at;
+    auto add = [&](const double* src, size_t n, const double** out) {
+        at.push_back({out, tables.size()});
+        tables.insert(tables.end(), src, src + n);
+        tables.resize((tables.size() + 31) & ~size_t(31), 0.0);
     };
-    int rc = 0;
-    for (int k = 0; k < d.ndim && !rc; ++k) {
-        rc = up(hg->ax[k].x, hg->ax[k].n, &dg->ax[k].x);
-        if (!rc) rc = up(hg->ax[k].inc, hg->ax[k].n, &dg->ax[k].inc);
-        if (!rc && hg->unrolled != GRID_GENERAL) rc = up(lin[k].data(), lin[k].size(), &dg->ax[k].lin);
+    for (int k = 0; k < d.ndim; ++k) {
+        add(hg->ax[k].x, hg->ax[k].n, &dg->ax[k].x);
+        add(hg->ax[k].inc, hg->ax[k].n, &dg->ax[k].inc);
+        if (hg->unrolled != GRID_GENERAL) add(lin[k].data(), lin[k].size(), &dg->ax[k].lin);
     }
-    if (!rc && hg->unrolled == GRID_PCHIP0) rc = up(pch.data(), pch.size(), &dg->ax[0].pch);
-    if (!rc) rc = up(hg->data, total, &dg->data);
+    if (hg->unrolled == GRID_PCHIP0) add(pch.data(), pch.size(), &dg->ax[0].pch);
+    const size_t nt = tables.size();
+    void* mem = nullptr;
+    cudaError_t e = cudaMalloc(&mem, (nt + total) * sizeof(double));
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        wq3d_internal_release_idle();
+        e = cudaMalloc(&mem, (nt + total) * sizeof(double));
+    }
+    WQ_CK(e);
+    o->dmem.push_back(mem);
+    double* base = static_cast<double*>(mem);
+    for (const auto& f : at) *f.first = base + f.second;
+    dg->data = base + nt;
+    WQ_CK(cudaMemcpy(base, tables.data(), nt * sizeof(double), cudaMemcpyHostToDevice));
+    WQ_CK(cudaMemcpy(base + nt, hg->data, total * sizeof(double), cudaMemcpyHostToDevice));
     /* a queue's streams do not wait for the default stream's copies */
-    if (!rc) WQ_CK(cudaStreamSynchronize(cudaStreamLegacy));
-    return rc;
+    WQ_CK(cudaStreamSynchronize(cudaStreamLegacy));
+    return WQ3D_OK;
 }
 
 }  // namespace
@@ -793,11 +799,17 @@ struct wq3d_queue : QueueRt {
     }
 
     /* A record buffer's capacity for "need" records of rec_bytes each: at
-     * least 4096, at most a quarter of the free device memory. */
+     * least 4096, at most a quarter of the free device memory.  What the
+     * pool holds idle does not count, since it may lie in pieces too small
+     * for the buffer; it is given back first when the rest is short. */
     int record_capacity(size_t need, size_t rec_bytes, size_t* out) {
         size_t free_b = 0, total_b = 0;
         WQ_CK(cudaMemGetInfo(&free_b, &total_b));
-        free_b += pool_idle_bytes(device);
+        if ((free_b / 4) / rec_bytes < need) {
+            WQ_CK(cudaStreamSynchronize(stream));
+            trim_pools();
+            WQ_CK(cudaMemGetInfo(&free_b, &total_b));
+        }
         const size_t limit = std::max<size_t>(4096, (free_b / 4) / rec_bytes);
         *out = std::min<size_t>({std::max<size_t>(need, 4096), limit, (size_t)UINT32_MAX / 2});
         return WQ3D_OK;
@@ -884,9 +896,12 @@ struct wq3d_queue : QueueRt {
         WQ_CK(device_pool(device, &pool));
         cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool, stream);
         if (e == cudaErrorMemoryAllocation) {
+            /* the stream's own releases must have run to be given back */
             cudaGetLastError();
-            cudaMemPoolTrimTo(pool, 0);
+            WQ_CK(cudaStreamSynchronize(stream));
+            wq3d_internal_release_idle();
             e = cudaMallocFromPoolAsync(&p, bytes, pool, stream);
+            if (e != cudaSuccess) cudaGetLastError(); /* not the next call's error */
         }
         if (e != cudaSuccess) return fail(WQ3D_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
         allocs.push_back(p);
@@ -1680,6 +1695,19 @@ wq3d_queue* cache_take(int device, size_t nde, size_t naz, size_t nf, size_t nt1
     return nullptr;
 }
 }  // namespace
+
+void wq3d_internal_release_idle(void) {
+    std::vector<wq3d_queue*> drop;
+    {
+        std::lock_guard<std::mutex> lock(g_cache_mu);
+        drop.swap(*g_cache);
+    }
+    for (wq3d_queue* q : drop) {
+        DeviceGuard guard(q->device);
+        delete q;
+    }
+    trim_pools();
+}
 
 int wq3d_set_queue_cache(size_t max_queues) {
     std::vector<wq3d_queue*> drop;

@@ -43,6 +43,7 @@
 #include "wq3d.h"
 
 extern "C" void wq3d_internal_set_error(const char* msg);
+extern "C" void wq3d_internal_release_idle(void);
 
 namespace {
 
@@ -393,8 +394,14 @@ struct BvWorkspace {
             p[k] = nullptr;
             cap[k] = 0;
             const size_t want = bytes + bytes / 4;
-            const cudaError_t e = cudaMalloc(&p[k], want);
+            cudaError_t e = cudaMalloc(&p[k], want);
+            if (e == cudaErrorMemoryAllocation) { /* what destroyed queues left */
+                cudaGetLastError();
+                wq3d_internal_release_idle();
+                e = cudaMalloc(&p[k], want);
+            }
             if (e != cudaSuccess) {
+                cudaGetLastError();
                 p[k] = nullptr;
                 return e;
             }

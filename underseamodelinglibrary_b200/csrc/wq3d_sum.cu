@@ -22,6 +22,7 @@
 using namespace wq3d;
 
 extern "C" void wq3d_internal_set_error(const char* msg);
+extern "C" void wq3d_internal_release_idle(void);
 
 namespace {
 
@@ -135,6 +136,11 @@ extern "C" int wq3d_sum_eigenrays(const wq3d_eigenray* rays, const double* inten
     const size_t b_tot = al(nt * sizeof(SumRay)), b_ti = al(nt * nf * 8);
     const size_t bytes = b_first + b_order + b_rays + 2 * b_in + b_freq + b_tot + 2 * b_ti;
     cudaError_t e = cudaMalloc(&dmem, bytes);
+    if (e == cudaErrorMemoryAllocation) { /* what destroyed queues left */
+        cudaGetLastError();
+        wq3d_internal_release_idle();
+        e = cudaMalloc(&dmem, bytes);
+    }
     if (e != cudaSuccess) return sum_fail(WQ3D_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     char* p = dmem;
     auto take = [&](size_t b) {
