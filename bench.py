@@ -43,9 +43,10 @@ FLOPS_PER_RAY_TARGET_STEP = 17
 # FP64 bytes the CPA kernel must read per interior ray and launch: four
 # distance2 terms (rho, theta, phi, sin theta) on three fronts plus on_edge
 BYTES_PER_RAY_CPA = 3 * 4 * 8 + 1
-# dram__bytes_read.sum + dram__bytes_write.sum of one k_cpa_f32 launch on
-# this workload (ncu, launch 301; profiles/fp32c_step_kernels_*.md)
-NCU_TRAFFIC_CPA_F32 = 15986688 + 0
+# dram__bytes_read.sum + dram__bytes_write.sum of one k_cpa and one
+# k_cpa_items launch on this workload (ncu, step 360;
+# profiles/search_step_kernels_*.md)
+NCU_TRAFFIC_CPA = 13086720 + 17664
 
 
 def parse():
@@ -99,6 +100,10 @@ class ClockSampler:
             self.thread.start()
         except (OSError, FileNotFoundError):
             self.proc = None
+
+    def sampling(self):
+        """the first sample is there, or none will come"""
+        return self.proc is None or self.proc.poll() is not None or bool(self.lines)
 
     def _read(self):
         for line in self.proc.stdout:
@@ -253,6 +258,15 @@ def engine_arm(args, rank, world, dist):
         del q
     clocks = ClockSampler(rank)
     clocks.start()
+    # nvidia-smi's own start takes the driver's locks and holds up the capture
+    # of a queue's graphs (138 ms a propagation in one run, 66-72 otherwise),
+    # so untimed propagations go on until it has given its first sample
+    t_wait = time.perf_counter()
+    while not clocks.sampling() and time.perf_counter() - t_wait < 5.0:
+        q = make()
+        q.run(sc["time_max"])
+        q.take_eigenrays()
+        del q
     if dist is not None:
         dist.barrier()
     total_ms, launches, n_eig = timed_runs(_abi.FP32C, args.steps)
@@ -330,9 +344,9 @@ def engine_arm(args, rank, world, dist):
                      "peak": fp32_peak,
                      "unit": "TFLOP/s",
                      "frac": (achieved / fp32_peak) if fp32_peak else None,
-                     "traffic": NCU_TRAFFIC_CPA_F32,
+                     "traffic": NCU_TRAFFIC_CPA,
                      "traffic_unit": "bytes per launch (ncu capture)",
-                     "kernel": "k_cpa_f32",
+                     "kernel": "k_cpa + k_cpa_items",
                      "peak_source": "clock-derived: 148 SMs x 128 FP32 lanes x 2 x median SM clock %.0f MHz "
                                     "(MEASURED_PEAKS.json has no FP32/FP64 CUDA-core figure)" % sm_mhz,
                      "fp32_fma_loop_tflops": peaks["fp32"],

@@ -555,7 +555,7 @@ typedef struct wq3d_timing {
                             included                                    */
     double ms_advance;   /* k_advance (and k_volume), timing mode only  */
     double ms_reflect;   /* k_reflect on its side stream, timing mode only */
-    double ms_cpa;       /* k_cpa / k_cpa_f32, timing mode only          */
+    double ms_cpa;       /* k_cpa and k_cpa_items, timing mode only      */
     double ms_eigenray;  /* k_eigenray, timing mode only                 */
     int64_t launches;    /* kernel launches                              */
 } wq3d_timing;
