@@ -234,7 +234,8 @@ enum { WQ3D_CLASSIC_RAY = 0, WQ3D_HYBRID_GAUSSIAN = 1 }; /* wave_queue.h:90 */
 /* Arithmetic form.  WQ3D_FP64: the reference's FP64 arithmetic throughout.
  * WQ3D_FP32C: the same, with the CPA search's comparisons screened in FP32
  * and finished in FP64 where the screen cannot decide (the eigenrays equal
- * the FP64 form's bit for bit).  WQ3D_FP32: additionally the sound speed,
+ * the FP64 arithmetic's bit for bit, so WQ3D_FP64 queues are searched the
+ * same way, but in the bounds-checked build).  WQ3D_FP32: additionally the sound speed,
  * its gradient and the ray derivatives of every wave_front::update
  * (wave_front.cc:125-178) in FP32, at the altitude offset rho - R, while
  * positions, directions, travel time, the distance terms and the CPA
