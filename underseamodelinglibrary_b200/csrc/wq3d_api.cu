@@ -322,111 +322,6 @@ int make_grid(wq3d_ocean* o, const wq3d_grid_desc& d, int max_dims, GridDev* hg,
 
 namespace {
 
-/* the CPA search's view of the targets (QueueDev::clusters, cpa_tgt,
- * cpa_index, tgt_box) */
-struct CpaTargets {
-    std::vector<TgtCluster> clusters;
-    std::vector<double> tgt;
-    std::vector<uint32_t> index;
-    double box[6] = {0, 0, 0, 0, 0, 0};
-};
-
-/* the clusters of the targets in the given order, and the sum of their
- * extents in metres */
-double make_clusters(const std::vector<double>& r, const std::vector<double>& th, const std::vector<double>& ph,
-                     const std::vector<double>& sn, const std::vector<uint8_t>& branch,
-                     const std::vector<uint32_t>& order, std::vector<TgtCluster>* out) {
-    out->clear();
-    double total = 0.0;
-    for (size_t b = 0; b < order.size(); b += 32) {
-        const size_t e = std::min(order.size(), b + 32);
-        double lo[4], hi[4];
-        for (size_t j = b; j < e; ++j) {
-            const uint32_t t = order[j];
-            const double v[4] = {r[t], th[t], ph[t], r[t] * sn[t]};
-            for (int k = 0; k < 4; ++k) {
-                /* a NaN stays, and makes the cluster's bounds NaN */
-                if (j == b || !(v[k] >= lo[k])) lo[k] = v[k];
-                if (j == b || !(v[k] <= hi[k])) hi[k] = v[k];
-            }
-        }
-        TgtCluster c{};
-        for (size_t j = b; j < e; ++j) c.branch |= branch[order[j]];
-        double mid[4], half[4];
-        for (int k = 0; k < 4; ++k) {
-            mid[k] = 0.5 * (lo[k] + hi[k]);
-            half[k] = std::max(hi[k] - mid[k], mid[k] - lo[k]) * 1.000001;
-        }
-        c.R = mid[0];
-        c.T = mid[1];
-        c.P = mid[2];
-        c.RS = mid[3];
-        c.dR = (float)half[0];
-        c.dT = (float)half[1];
-        c.dP = (float)half[2];
-        c.dRS = (float)half[3];
-        total += half[0] + std::abs(mid[0]) * half[1] + std::abs(mid[3]) * half[2];
-        out->push_back(c);
-    }
-    return total;
-}
-
-/* Clusters of 32 consecutive targets, in the caller's order or along a
- * Morton curve, whichever has the smaller extents: a range x depth table's
- * columns are already compact (1.5 of 32 clusters survive a warp's bounds on
- * the sloped workload, 3 along the curve), random targets are not (27 of 128
- * on the reverberation workload, 126 in their own order). */
-void cpa_targets(const std::vector<double>& r, const std::vector<double>& th, const std::vector<double>& ph,
-                 const std::vector<double>& sn, const std::vector<uint8_t>& branch, CpaTargets* o) {
-    const size_t nt = r.size();
-    o->index.resize(nt);
-    for (size_t t = 0; t < nt; ++t) o->index[t] = (uint32_t)t;
-    double lo[3], hi[3];
-    for (size_t t = 0; t < nt; ++t) {
-        const double v[3] = {r[t], th[t], ph[t]};
-        for (int k = 0; k < 3; ++k) {
-            if (t == 0 || !(v[k] >= lo[k])) lo[k] = v[k];
-            if (t == 0 || !(v[k] <= hi[k])) hi[k] = v[k];
-        }
-    }
-    for (int k = 0; k < 3 && nt; ++k) {
-        o->box[2 * k] = lo[k];
-        o->box[2 * k + 1] = hi[k];
-    }
-    const double own = make_clusters(r, th, ph, sn, branch, o->index, &o->clusters);
-    if (nt > 32) {
-        const double size = std::max({hi[0] - lo[0], hi[0] * (hi[1] - lo[1]), hi[0] * (hi[2] - lo[2])});
-        if (size > 0.0 && size < 1e30) {
-            std::vector<std::pair<uint64_t, uint32_t>> key(nt);
-            for (size_t t = 0; t < nt; ++t) {
-                const double x[3] = {r[t] - lo[0], hi[0] * (th[t] - lo[1]), hi[0] * sn[t] * (ph[t] - lo[2])};
-                uint64_t m = 0;
-                for (int k = 0; k < 3; ++k) {
-                    const uint32_t c = (uint32_t)std::min(1023.0, std::max(0.0, 1023.0 * x[k] / size));
-                    for (int b = 0; b < 10; ++b) m |= (uint64_t)((c >> b) & 1u) << (3 * b + k);
-                }
-                key[t] = {m, (uint32_t)t};
-            }
-            std::sort(key.begin(), key.end());
-            std::vector<uint32_t> order(nt);
-            for (size_t t = 0; t < nt; ++t) order[t] = key[t].second;
-            std::vector<TgtCluster> cl;
-            if (make_clusters(r, th, ph, sn, branch, order, &cl) < own) {
-                o->index.swap(order);
-                o->clusters.swap(cl);
-            }
-        }
-    }
-    o->tgt.resize(4 * nt);
-    for (size_t j = 0; j < nt; ++j) {
-        const uint32_t t = o->index[j];
-        o->tgt[4 * j] = r[t];
-        o->tgt[4 * j + 1] = th[t];
-        o->tgt[4 * j + 2] = ph[t];
-        o->tgt[4 * j + 3] = sn[t];
-    }
-}
-
 /* The patches of rays that CPA warps take: bands of 32, 16, 8, 4, 2 or 1
  * D/E rows cut along AZ.  A band's shape keeps the angular extents of its
  * patches smallest: its D/E span against half the AZ span, times the cosine
@@ -1892,8 +1787,9 @@ int wq3d_queue_create(const wq3d_ocean* ocean, const wq3d_queue_desc* d, wq3d_qu
     CpaTargets cpa;
     cpa_targets(tr, tt, tp, tsin, tbranch, &cpa);
     std::copy(cpa.box, cpa.box + 6, h.tgt_box);
+    h.n_cpa_tgt = (int)cpa.index.size();
     std::vector<CpaPatch> patches;
-    if (nt) cpa_patches(de, az, nt, &patches);
+    if (!cpa.index.empty()) cpa_patches(de, az, cpa.index.size(), &patches);
     h.n_patch = (int)patches.size();
     /* spreading normalisation (spreading_hybrid_gaussian.cc:28-59,
      * spreading_ray.cc:26-45) */

@@ -28,6 +28,7 @@
 #include <stdint.h>
 
 #include "wq3d_models.cuh"
+#include "wq3d_targets.h"
 
 namespace wq3d {
 
@@ -115,15 +116,6 @@ struct CpaPatch {
     uint8_t shift, part, parts, pad[3];
 };
 
-/* 32 targets of the CPA search: the middle of their ranges of rho, theta,
- * phi and rho sin(theta), and the half-widths (rounded up) */
-struct TgtCluster {
-    double R, T, P, RS;
-    float dR, dT, dP, dRS;
-    int32_t branch; /* holds a target with QueueDev::de_branch set */
-    int32_t pad;
-};
-
 struct FrontPtrs {
     double* pos[3];
     double* pg[3];
@@ -181,9 +173,10 @@ struct QueueDev {
     const uint8_t* de_branch;
     /* the CPA search's targets, in clusters of 32 that lie near one another */
     const TgtCluster* clusters;
-    const double* cpa_tgt;       /* [nt][4] rho, theta, phi, sin(theta) */
-    const uint32_t* cpa_index;   /* [nt] index of each in the arrays above */
-    double tgt_box[6];           /* least and largest rho, theta, phi   */
+    const double* cpa_tgt;       /* [n_cpa_tgt][4] rho, theta, phi, sin(theta) */
+    const uint32_t* cpa_index;   /* [n_cpa_tgt] index of each in the arrays above */
+    int n_cpa_tgt;               /* the targets with finite coordinates */
+    double tgt_box[6];           /* their least and largest rho, theta, phi */
     const CpaPatch* patches;     /* [n_patch] work of each CPA warp     */
     int n_patch;
     uint4* items;                /* [cap_item] (patch, target, rays) left by k_cpa */

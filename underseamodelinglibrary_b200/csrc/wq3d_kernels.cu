@@ -1525,7 +1525,8 @@ __device__ __forceinline__ bool is_closest(const QueueDev& q, const FrontPtrs& V
  * 192 u where a cluster's extents enter.  All add c0 = max(1 m^2, 4e-15 (rho^2 + R^2)) for
  * the rounding of the reference's FP64 expression on the two points (each
  * within 5 x 2^-53 (rho^2 + R^2), 0.05 m^2 at earth radius).  A NaN in a ray
- * or target makes its bounds NaN, which reject nothing.
+ * makes its patch's bounds NaN, which reject nothing; targets with a NaN or
+ * infinite coordinate are not searched (cpa_targets).
  *
  * Why this shape: per pair the search costs what the bounds let through.
  * On the sloped workload (1801 x 91 rays, 1024 targets, step 100) the two
@@ -1773,7 +1774,7 @@ __global__ void __launch_bounds__(32 * CPA_WARPS, 4) k_cpa(__grid_constant__ con
     }
     __syncwarp();
     /* this warp's share of the clusters; nothing more to do for most warps */
-    const int ncl = (q.nt + 31) >> 5;
+    const int ncl = (q.n_cpa_tgt + 31) >> 5;
     const int per = (ncl + P.parts - 1) / P.parts;
     const int c_begin = P.part * per, c_end = min(ncl, c_begin + per);
     {
@@ -1821,9 +1822,9 @@ __global__ void __launch_bounds__(32 * CPA_WARPS, 4) k_cpa(__grid_constant__ con
     };
 #if WQ3D_CHECKED
     if (q.precision == WQ3D_FP64) {
-        for (int j0 = c_begin * 32; j0 < min(q.nt, c_end * 32); j0 += 32) {
+        for (int j0 = c_begin * 32; j0 < min(q.n_cpa_tgt, c_end * 32); j0 += 32) {
             const int j = j0 + lane;
-            append(j < q.nt, j < q.nt ? q.cpa_index[j] : 0u, 0xffffffffu);
+            append(j < q.n_cpa_tgt, j < q.n_cpa_tgt ? q.cpa_index[j] : 0u, 0xffffffffu);
         }
         return;
     }
@@ -1870,7 +1871,7 @@ __global__ void __launch_bounds__(32 * CPA_WARPS, 4) k_cpa(__grid_constant__ con
                 cmask &= cmask - 1;
                 bool want = false;
                 uint32_t t = 0;
-                if (j < q.nt) {
+                if (j < q.n_cpa_tgt) {
                     const double2 a = __ldg(reinterpret_cast<const double2*>(q.cpa_tgt) + 2 * (size_t)j);
                     const double2 b = __ldg(reinterpret_cast<const double2*>(q.cpa_tgt) + 2 * (size_t)j + 1);
                     t = __ldg(q.cpa_index + j);
