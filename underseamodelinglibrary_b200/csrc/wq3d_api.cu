@@ -21,6 +21,7 @@
 #include <tuple>
 #include <vector>
 
+#include "wq3d_buffers.h"
 #include "wq3d_engine.cuh"
 
 using namespace wq3d;
@@ -709,32 +710,53 @@ struct wq3d_queue : QueueRt {
         *out = std::min<size_t>({std::max<size_t>(need, 4096), limit, (size_t)UINT32_MAX / 2});
         return WQ3D_OK;
     }
-    template <class T>
-    int remake(T** p, size_t count) {
-        release(*p);
-        *p = nullptr;
-        return alloc(p, count);
+    /* buffers[k].fresh: all of the new buffers, or none and an error */
+    int make_buffers(std::vector<Resize>& buffers) {
+        return make_all(
+            buffers,
+            [&](void** out, size_t bytes) {
+                char* p = nullptr;
+                const int rc = alloc(&p, bytes);
+                *out = p;
+                return rc;
+            },
+            [&](void* p) { release(p); });
+    }
+    /* the same for record buffers, whose addresses the chunk graphs hold:
+     * the graphs go before the old buffers do */
+    int grow_buffers(std::vector<Resize>& buffers) {
+        WQ_CK(cudaStreamSynchronize(stream));
+        const int rc = make_buffers(buffers);
+        if (rc) return rc;
+        drop_graph();
+        for (const Resize& b : buffers) release(b.old);
+        return WQ3D_OK;
     }
 
     /* Eigenverb buffers (both result sets) hold at least "need" records.
      * They start at half a record per ray, step and interface of a chunk
      * and grow when a chunk fills more than half of them.  Runs with no
-     * chunk in flight; drops the graphs, which hold the pointers. */
+     * chunk in flight; when it fails the queue keeps the buffers it had. */
     int ensure_verb_capacity(size_t need) {
         if (h.verb && need <= h.cap_verb) return WQ3D_OK;
         size_t cap = 0;
         int rc = record_capacity(need, sizeof(wq3d_eigenverb) + (size_t)h.nf * sizeof(double), &cap);
         if (rc) return rc;
         if (h.verb && cap <= h.cap_verb) return WQ3D_OK;
-        WQ_CK(cudaStreamSynchronize(stream));
-        h.cap_verb = 0;
-        rc = remake(&h.verb, cap);
-        if (!rc) rc = remake(&h.verb_power, cap * (size_t)h.nf);
-        if (!rc && have_set1) rc = remake(&set1.verb, cap);
-        if (!rc && have_set1) rc = remake(&set1.verb_power, cap * (size_t)h.nf);
-        if (rc) return rc;
+        const size_t rec_b = cap * sizeof(wq3d_eigenverb), pow_b = cap * (size_t)h.nf * sizeof(double);
+        std::vector<Resize> b{{h.verb, rec_b, nullptr}, {h.verb_power, pow_b, nullptr}};
+        if (have_set1) {
+            b.push_back({set1.verb, rec_b, nullptr});
+            b.push_back({set1.verb_power, pow_b, nullptr});
+        }
+        if ((rc = grow_buffers(b))) return rc;
+        h.verb = static_cast<wq3d_eigenverb*>(b[0].fresh);
+        h.verb_power = static_cast<double*>(b[1].fresh);
+        if (have_set1) {
+            set1.verb = static_cast<wq3d_eigenverb*>(b[2].fresh);
+            set1.verb_power = static_cast<double*>(b[3].fresh);
+        }
         h.cap_verb = (uint32_t)cap;
-        drop_graph();
         return WQ3D_OK;
     }
 
@@ -746,13 +768,12 @@ struct wq3d_queue : QueueRt {
         int rc = record_capacity(need, sizeof(wq3d_reflection), &cap);
         if (rc) return rc;
         if (cap <= h.cap_refl) return WQ3D_OK;
-        WQ_CK(cudaStreamSynchronize(stream));
-        h.cap_refl = 0;
-        rc = remake(&h.refl, cap);
-        if (!rc && have_set1) rc = remake(&set1.refl, cap);
-        if (rc) return rc;
+        std::vector<Resize> b{{h.refl, cap * sizeof(wq3d_reflection), nullptr}};
+        if (have_set1) b.push_back({set1.refl, cap * sizeof(wq3d_reflection), nullptr});
+        if ((rc = grow_buffers(b))) return rc;
+        h.refl = static_cast<wq3d_reflection*>(b[0].fresh);
+        if (have_set1) set1.refl = static_cast<wq3d_reflection*>(b[1].fresh);
         h.cap_refl = (uint32_t)cap;
-        drop_graph();
         return WQ3D_OK;
     }
 
