@@ -2421,15 +2421,28 @@ static int adjoint_sweep(wq3d_queue* q, const wq3d_eigenray* rays, const double*
     auto& W = q->adjw;
     int rc = WQ3D_OK;
     if (!W.seg) {
-        if ((rc = q->alloc(&W.seg, (size_t)(K + 1) * ADJ_S * n)) || (rc = q->alloc(&W.chain, (size_t)(K + 1) * n)) ||
-            (rc = q->alloc(&W.seed, (size_t)(K + 1) * ADJ_L * n)) || (rc = q->alloc(&W.lam, (size_t)ADJ_L * n)) ||
-            (rc = q->alloc(&W.last, n)) || (rc = q->alloc(&W.grad, ADJ_MAX_NODES)) || (rc = q->alloc(&W.err, 1)))
-            return rc;
+        const size_t d8 = sizeof(double);
+        std::vector<Resize> b{{nullptr, (size_t)(K + 1) * ADJ_S * n * d8, nullptr},
+                              {nullptr, (size_t)(K + 1) * n * sizeof(uint32_t), nullptr},
+                              {nullptr, (size_t)(K + 1) * ADJ_L * n * d8, nullptr},
+                              {nullptr, (size_t)ADJ_L * n * d8, nullptr},
+                              {nullptr, n * sizeof(int64_t), nullptr},
+                              {nullptr, ADJ_MAX_NODES * d8, nullptr},
+                              {nullptr, sizeof(uint32_t), nullptr}};
+        if ((rc = q->make_buffers(b))) return rc;
+        W.seg = static_cast<double*>(b[0].fresh);
+        W.chain = static_cast<uint32_t*>(b[1].fresh);
+        W.seed = static_cast<double*>(b[2].fresh);
+        W.lam = static_cast<double*>(b[3].fresh);
+        W.last = static_cast<int64_t*>(b[4].fresh);
+        W.grad = static_cast<double*>(b[5].fresh);
+        W.err = static_cast<uint32_t*>(b[6].fresh);
     }
     if (W.w_cap < 2 * (size_t)nrec) {
+        std::vector<Resize> b{{W.w, std::max<size_t>(2 * (size_t)nrec, 2) * sizeof(double), nullptr}};
+        if ((rc = q->make_buffers(b))) return rc;
         q->release(W.w);
-        W.w = nullptr;
-        if ((rc = q->alloc(&W.w, std::max<size_t>(2 * (size_t)nrec, 2)))) return rc;
+        W.w = static_cast<double*>(b[0].fresh);
         W.w_cap = std::max<size_t>(2 * (size_t)nrec, 2);
     }
     cudaStream_t st = q->stream;
