@@ -192,6 +192,27 @@ void trim_pools() {
  * what the pools hold idle */
 extern "C" void wq3d_internal_release_idle(void);
 
+namespace {
+/* cudaMalloc, with what destroyed queues left given back when it finds no
+ * room.  A failure is the caller's to report: it is not left for the
+ * runtime's next error query, which queue creation makes. */
+template <class T>
+cudaError_t device_malloc(T** out, size_t count) {
+    const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
+    cudaError_t e = cudaMalloc(out, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        wq3d_internal_release_idle();
+        e = cudaMalloc(out, bytes);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        *out = nullptr;
+    }
+    return e;
+}
+}  // namespace
+
 struct wq3d_ocean {
     OceanDev dev;   /* device pointers, passed to kernels        */
     OceanDev host;  /* host pointers, for host-side evaluations  */
@@ -300,16 +321,9 @@ int make_grid(wq3d_ocean* o, const wq3d_grid_desc& d, int max_dims, GridDev* hg,
     }
     if (hg->unrolled == GRID_PCHIP0) add(pch.data(), pch.size(), &dg->ax[0].pch);
     const size_t nt = tables.size();
-    void* mem = nullptr;
-    cudaError_t e = cudaMalloc(&mem, (nt + total) * sizeof(double));
-    if (e == cudaErrorMemoryAllocation) {
-        cudaGetLastError();
-        wq3d_internal_release_idle();
-        e = cudaMalloc(&mem, (nt + total) * sizeof(double));
-    }
-    WQ_CK(e);
-    o->dmem.push_back(mem);
-    double* base = static_cast<double*>(mem);
+    double* base = nullptr;
+    WQ_CK(device_malloc(&base, nt + total));
+    o->dmem.push_back(base);
     for (const auto& f : at) *f.first = base + f.second;
     dg->data = base + nt;
     WQ_CK(cudaMemcpy(base, tables.data(), nt * sizeof(double), cudaMemcpyHostToDevice));
@@ -1459,7 +1473,7 @@ int wq3d_ocean_destroy(wq3d_ocean* o) {
 static int eval_points(size_t n, std::vector<double*>& dev_in, const std::vector<const double*>& host_in) {
     for (size_t k = 0; k < host_in.size(); ++k) {
         double* p = nullptr;
-        WQ_CK(cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(double)));
+        WQ_CK(device_malloc(&p, n));
         dev_in.push_back(p);
         if (host_in[k])
             WQ_CK(cudaMemcpy(p, host_in[k], n * sizeof(double), cudaMemcpyHostToDevice));
@@ -1476,8 +1490,8 @@ int wq3d_ocean_sound_speed(const wq3d_ocean* o, double R, size_t n, const double
     std::vector<double*> d;
     int rc = eval_points(n, d, {rho, theta, phi});
     double *dc = nullptr, *dg = nullptr;
-    if (!rc && cudaMalloc(&dc, std::max<size_t>(n, 1) * sizeof(double)) != cudaSuccess) rc = WQ3D_ERR_CUDA;
-    if (!rc && cudaMalloc(&dg, std::max<size_t>(3 * n, 1) * sizeof(double)) != cudaSuccess) rc = WQ3D_ERR_CUDA;
+    if (!rc && device_malloc(&dc, n) != cudaSuccess) rc = WQ3D_ERR_CUDA;
+    if (!rc && device_malloc(&dg, 3 * n) != cudaSuccess) rc = WQ3D_ERR_CUDA;
     if (!rc && n > 0) {
         k_sound_speed<<<(unsigned)((n + 127) / 128), 128>>>(o->dev, R, (int)n, d[0], d[1], d[2], dc, dg);
         if (cudaMemcpy(speed, dc, n * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess) rc = WQ3D_ERR_CUDA;
@@ -1499,8 +1513,8 @@ int wq3d_ocean_height(const wq3d_ocean* o, int which, size_t n, const double* rh
     std::vector<double*> d;
     int rc = eval_points(n, d, {theta, phi});
     double *dh = nullptr, *dn = nullptr;
-    if (!rc && cudaMalloc(&dh, std::max<size_t>(n, 1) * sizeof(double)) != cudaSuccess) rc = WQ3D_ERR_CUDA;
-    if (!rc && cudaMalloc(&dn, std::max<size_t>(3 * n, 1) * sizeof(double)) != cudaSuccess) rc = WQ3D_ERR_CUDA;
+    if (!rc && device_malloc(&dh, n) != cudaSuccess) rc = WQ3D_ERR_CUDA;
+    if (!rc && device_malloc(&dn, 3 * n) != cudaSuccess) rc = WQ3D_ERR_CUDA;
     if (!rc && n > 0) {
         k_height<<<(unsigned)((n + 127) / 128), 128>>>(which == 0 ? o->dev.surf : o->dev.bot, (int)n, d[0],
                                                         d[1], dh, dn);
@@ -1525,9 +1539,9 @@ int wq3d_ocean_attenuation(const wq3d_ocean* o, double earth_radius, size_t n, c
     std::vector<double*> d;
     int rc = eval_points(n, d, {rho, distance});
     double *df = nullptr, *dal = nullptr, *da = nullptr;
-    if (!rc && cudaMalloc(&df, nf * sizeof(double)) != cudaSuccess) rc = WQ3D_ERR_CUDA;
-    if (!rc && cudaMalloc(&dal, nf * sizeof(double)) != cudaSuccess) rc = WQ3D_ERR_CUDA;
-    if (!rc && cudaMalloc(&da, n * nf * sizeof(double)) != cudaSuccess) rc = WQ3D_ERR_CUDA;
+    if (!rc && device_malloc(&df, nf) != cudaSuccess) rc = WQ3D_ERR_CUDA;
+    if (!rc && device_malloc(&dal, nf) != cudaSuccess) rc = WQ3D_ERR_CUDA;
+    if (!rc && device_malloc(&da, n * nf) != cudaSuccess) rc = WQ3D_ERR_CUDA;
     if (!rc && cudaMemcpy(df, freq, nf * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) rc = WQ3D_ERR_CUDA;
     if (!rc && cudaMemcpy(dal, alpha.data(), nf * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
         rc = WQ3D_ERR_CUDA;
@@ -1557,9 +1571,9 @@ int wq3d_ocean_reflect_loss(const wq3d_ocean* o, int which, size_t n, const doub
     std::vector<double*> d;
     int rc = eval_points(n, d, {grazing});
     double *df = nullptr, *da = nullptr, *dp = nullptr;
-    if (!rc && cudaMalloc(&df, std::max<size_t>(nf, 1) * sizeof(double)) != cudaSuccess) rc = WQ3D_ERR_CUDA;
-    if (!rc && cudaMalloc(&da, std::max<size_t>(n * nf, 1) * sizeof(double)) != cudaSuccess) rc = WQ3D_ERR_CUDA;
-    if (!rc && cudaMalloc(&dp, std::max<size_t>(n * nf, 1) * sizeof(double)) != cudaSuccess) rc = WQ3D_ERR_CUDA;
+    if (!rc && device_malloc(&df, nf) != cudaSuccess) rc = WQ3D_ERR_CUDA;
+    if (!rc && device_malloc(&da, n * nf) != cudaSuccess) rc = WQ3D_ERR_CUDA;
+    if (!rc && device_malloc(&dp, n * nf) != cudaSuccess) rc = WQ3D_ERR_CUDA;
     if (!rc && n > 0) {
         cudaMemcpy(df, freq, nf * sizeof(double), cudaMemcpyHostToDevice);
         k_reflect_loss<<<(unsigned)((n + 127) / 128), 128>>>(which == 0 ? o->dev.surf : o->dev.bot, (int)n,

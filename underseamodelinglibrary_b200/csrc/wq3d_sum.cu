@@ -141,7 +141,10 @@ extern "C" int wq3d_sum_eigenrays(const wq3d_eigenray* rays, const double* inten
         wq3d_internal_release_idle();
         e = cudaMalloc(&dmem, bytes);
     }
-    if (e != cudaSuccess) return sum_fail(WQ3D_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        cudaGetLastError(); /* not the next call's error */
+        return sum_fail(WQ3D_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    }
     char* p = dmem;
     auto take = [&](size_t b) {
         char* r = p;
