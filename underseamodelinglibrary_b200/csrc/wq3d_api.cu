@@ -685,12 +685,12 @@ struct wq3d_queue : QueueRt {
         const size_t nf = (size_t)h.nf;
         ResultSet s;
         const size_t before = allocs.size();
-        bool ok = !alloc(&s.rec, h.cap_rec) && !alloc(&s.rec_inten, (size_t)h.cap_rec * nf) &&
-                  !alloc(&s.rec_phase, (size_t)h.cap_rec * nf) && !alloc(&s.refl, h.cap_refl) &&
-                  (!h.sens || !alloc(&s.rec_sens, (size_t)h.cap_rec * 3)) &&
-                  (!h.verb || (!alloc(&s.verb, h.cap_verb) && !alloc(&s.verb_power, (size_t)h.cap_verb * nf)));
+        auto get = [&](auto** out, size_t count) { return alloc(out, count, false) == WQ3D_OK; };
+        const bool ok = get(&s.rec, h.cap_rec) && get(&s.rec_inten, (size_t)h.cap_rec * nf) &&
+                        get(&s.rec_phase, (size_t)h.cap_rec * nf) && get(&s.refl, h.cap_refl) &&
+                        (!h.sens || get(&s.rec_sens, (size_t)h.cap_rec * 3)) &&
+                        (!h.verb || (get(&s.verb, h.cap_verb) && get(&s.verb_power, (size_t)h.cap_verb * nf)));
         if (!ok) {
-            cudaGetLastError();
             while (allocs.size() > before) release(allocs.back());
             return false;
         }
@@ -817,9 +817,12 @@ struct wq3d_queue : QueueRt {
         }
     }
 
-    /* from the device's pool, ready for every stream when it returns */
+    /* From the device's pool, ready for every stream when it returns.  A
+     * buffer that the queue needs may take the place of the destroyed queues
+     * kept for reuse; one that it can do without (required = false) takes
+     * only memory that nobody holds, and leaves no error text. */
     template <class T>
-    int alloc(T** out, size_t count) {
+    int alloc(T** out, size_t count, bool required = true) {
         void* p = nullptr;
         const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
         cudaMemPool_t pool;
@@ -829,11 +832,17 @@ struct wq3d_queue : QueueRt {
             /* the stream's own releases must have run to be given back */
             cudaGetLastError();
             WQ_CK(cudaStreamSynchronize(stream));
-            wq3d_internal_release_idle();
+            if (required)
+                wq3d_internal_release_idle();
+            else
+                trim_pools();
             e = cudaMallocFromPoolAsync(&p, bytes, pool, stream);
             if (e != cudaSuccess) cudaGetLastError(); /* not the next call's error */
         }
-        if (e != cudaSuccess) return fail(WQ3D_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+        if (e != cudaSuccess) {
+            if (!required) return WQ3D_ERR_CUDA;
+            return fail(WQ3D_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+        }
         allocs.push_back(p);
         WQ_CK(cudaStreamSynchronize(stream));
         *out = static_cast<T*>(p);
