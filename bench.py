@@ -11,9 +11,10 @@ synthetic (generated, no data files).
 value: whole-job ray-steps/s with the workload resident in HBM, timed with
 CUDA events on the engine's stream around the 800 steps.  e2e: the same
 metric through the public API with host buffers (queue creation from host
-arrays, propagation, eigenray records read back).  roofline: the CPA kernel
-(the dominant kernel) in FP64 operations against an FP64 throughput peak
-measured on this GPU by bench.py itself.  cpu_baseline: the CPU oracle (a
+arrays, propagation, eigenray records read back).  roofline: the search
+kernels against HBM, by the bytes that a launch cannot do without; they are
+bound by latency, so search_pairs_per_s says what they get done.
+cpu_baseline: the CPU oracle (a
 restatement of the reference's CPU wave_queue) on a bounded sample.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
@@ -36,10 +37,6 @@ import numpy as np  # noqa: E402
 METRIC = "ray-steps/s"
 WORKLOAD = "linear_slope_rayleigh_1801x91_1024tgt_5f_dt0.05_40s"
 
-# algorithmic work of the CPA search per (ray, target) pair and step: the
-# reference's distance2 (wave_front.cc:222-236: 15 FP64 operations) plus the
-# two time comparisons of detect_eigenrays (wave_queue.cc:386-393)
-FLOPS_PER_RAY_TARGET_STEP = 17
 # FP64 bytes the CPA kernel must read per interior ray and launch: four
 # distance2 terms (rho, theta, phi, sin theta) on three fronts plus on_edge
 BYTES_PER_RAY_CPA = 3 * 4 * 8 + 1
@@ -135,62 +132,6 @@ class ClockSampler:
                 "reasons": sorted(reasons), "samples": len(sm)}
 
 
-# ---------------------------------------------------------------- FP64 peak
-PEAK_SRC = r"""
-#include <cuda_runtime.h>
-template <class T>
-__global__ void fma_peak(T* out, int iters) {
-    T a = threadIdx.x * (T)1e-3, b = (T)1.0000001, c = (T)0.9999999, d = blockIdx.x * (T)1e-6;
-    T e = a + (T)1, f = d + (T)2, g = a * (T)0.5, h = d * (T)0.25;
-    for (int i = 0; i < iters; ++i) {
-        a = a * b + c; d = d * b + c; e = e * b + c; f = f * b + c;
-        g = g * b + c; h = h * b + c;
-    }
-    out[blockIdx.x * blockDim.x + threadIdx.x] = a + d + e + f + g + h;
-}
-template <class T>
-float run(int iters) {
-    T* out; cudaMalloc(&out, 148 * 8 * 256 * sizeof(T));
-    cudaEvent_t x, y; cudaEventCreate(&x); cudaEventCreate(&y);
-    fma_peak<T><<<148 * 8, 256>>>(out, 100);
-    cudaEventRecord(x);
-    fma_peak<T><<<148 * 8, 256>>>(out, iters);
-    cudaEventRecord(y); cudaEventSynchronize(y);
-    float ms = 0; cudaEventElapsedTime(&ms, x, y);
-    cudaFree(out); cudaEventDestroy(x); cudaEventDestroy(y);
-    return ms;
-}
-extern "C" float run_peak64(int iters) { return run<double>(iters); }
-extern "C" float run_peak32(int iters) { return run<float>(iters); }
-"""
-
-
-def measure_fma_peaks():
-    """FP64 and FP32 FMA throughput (TFLOP/s, an FMA counted as 2 flops) of
-    this GPU: 6 independent FMA chains per thread, 148 x 8 blocks of 256
-    threads.  MEASURED_PEAKS.json carries only HBM and bf16 tensor figures."""
-    import ctypes as C
-    import tempfile
-    out = {"fp64": None, "fp32": None, "source": "measured by bench.py (FMA loop)"}
-    try:
-        d = tempfile.mkdtemp()
-        cu = os.path.join(d, "peak.cu")
-        so = os.path.join(d, "peak.so")
-        open(cu, "w").write(PEAK_SRC)
-        subprocess.check_call(["nvcc", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-shared",
-                               "-Xcompiler", "-fPIC", "-o", so, cu], stdout=subprocess.DEVNULL,
-                              stderr=subprocess.DEVNULL)
-        lib = C.CDLL(so)
-        for name, key, iters in (("run_peak64", "fp64", 20000), ("run_peak32", "fp32", 40000)):
-            fn = getattr(lib, name)
-            fn.restype = C.c_float
-            ms = fn(iters)
-            out[key] = 148 * 8 * 256 * iters * 6 * 2 / (ms / 1e3) / 1e12
-    except Exception as e:  # noqa: BLE001
-        out["source"] = "unavailable: %s" % e
-    return out
-
-
 # ---------------------------------------------------------------- engine arm
 def max_over_ranks(values, dist):
     """Each value's maximum over the ranks (every rank calls this once, in
@@ -258,9 +199,16 @@ def engine_arm(args, rank, world, dist):
         del q
     clocks = ClockSampler(rank)
     clocks.start()
-    # nvidia-smi's own start takes the driver's locks and holds up the capture
-    # of a queue's graphs (138 ms a propagation in one run, 66-72 otherwise),
-    # so untimed propagations go on until it has given its first sample
+    # The timed propagations are of queues that are all alive at once.  When
+    # more queues have graphs than ever before in the process, the driver
+    # stops to make room for some of them (1 to 3 propagations of the first 20
+    # took 140-150 ms, the others and all later ones 66-68), so as many queues
+    # run just long enough to have theirs.
+    qs = [make() for _ in range(args.steps)]
+    for q in qs:
+        q.step(96)
+        q.take_eigenrays()
+    del q, qs
     t_wait = time.perf_counter()
     while not clocks.sampling() and time.perf_counter() - t_wait < 5.0:
         q = make()
@@ -307,17 +255,7 @@ def engine_arm(args, rank, world, dist):
     value = world * args.steps * ray_steps / total_s
     e2e = world * args.steps * ray_steps / e2e_s
 
-    # roofline of the CPA kernel: algorithmic FP64 operations per launch
     interior = (nde - 2) * ((naz - 1) if _wraps(sc["az"]) else (naz - 2))
-    cpa_launch_s = (cpa_ms / 1000.0) / nsteps
-    flops_launch = FLOPS_PER_RAY_TARGET_STEP * interior * nt
-    achieved = flops_launch / cpa_launch_s / 1e12
-    peaks = measure_fma_peaks()
-    # the FP32 peak from the clock: 148 SMs x 128 FP32 lanes x 2 flops per
-    # FMA x the median SM clock sampled during the timed region
-    sm_mhz = (clk or {}).get("sm_mhz") or 1965.0
-    fp32_peak = 148 * 128 * 2 * sm_mhz * 1e6 / 1e12
-    fp64_peak_clock = 148 * 64 * 2 * sm_mhz * 1e6 / 1e12
     out = {
         "metric": METRIC, "value": value, "unit": "ray-steps/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup,
@@ -340,23 +278,11 @@ def engine_arm(args, rank, world, dist):
                       "errors_vs_fp64_form": f32_err},
         "eigenrays_per_propagation": n_eig / args.steps,
         "kernel_ms": kern,
-        "roofline": {"bound": "fp32", "achieved": achieved,
-                     "peak": fp32_peak,
-                     "unit": "TFLOP/s",
-                     "frac": (achieved / fp32_peak) if fp32_peak else None,
-                     "traffic": NCU_TRAFFIC_CPA,
-                     "traffic_unit": "bytes per launch (ncu capture)",
-                     "kernel": "k_cpa + k_cpa_items",
-                     "peak_source": "clock-derived: 148 SMs x 128 FP32 lanes x 2 x median SM clock %.0f MHz "
-                                    "(MEASURED_PEAKS.json has no FP32/FP64 CUDA-core figure)" % sm_mhz,
-                     "fp32_fma_loop_tflops": peaks["fp32"],
-                     "frac_of_fma_loop": (achieved / peaks["fp32"]) if peaks["fp32"] else None,
-                     "fp64_peak": fp64_peak_clock,
-                     "fp64_fma_loop_tflops": peaks["fp64"],
-                     "fp64_form_cpa_frac_of_fp64_peak": (
-                         flops_launch / (kern64["cpa"] / 1000.0 / nsteps) / 1e12 / fp64_peak_clock),
-                     "algorithmic_flops_per_launch": flops_launch},
-        "roofline_hbm": hbm_roofline(interior, cpa_launch_s),
+        "roofline": search_roofline(interior, cpa_ms / 1000.0 / nsteps),
+        # (ray, target) pairs decided; the bounds decide most of them by
+        # patches of rays and clusters of targets
+        "search_pairs_per_s": {"fp32c_form": interior * nt * nsteps / (cpa_ms / 1000.0),
+                               "fp64_form": interior * nt * nsteps / (kern64["cpa"] / 1000.0)},
         "clocks": clk,
     }
     if args.batch_instances > 0:
@@ -663,7 +589,7 @@ def _wraps(az):
     return math.fmod(a0 + 360.0, 360.0) == math.fmod(a1 + 360.0, 360.0)
 
 
-def hbm_roofline(interior, launch_s):
+def search_roofline(interior, launch_s):
     peaks = {}
     try:
         peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
@@ -674,7 +600,10 @@ def hbm_roofline(interior, launch_s):
     peak = peak or 6650.0
     achieved = interior * BYTES_PER_RAY_CPA / launch_s / 1e9
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-            "frac": achieved / peak, "traffic": None, "peak_source": src}
+            "frac": achieved / peak, "traffic": NCU_TRAFFIC_CPA,
+            "traffic_unit": "bytes per launch (ncu capture)", "peak_source": src,
+            "kernel": "k_cpa + k_cpa_items",
+            "limited_by": "latency: each warp reads its rays and forms their ranges once a launch"}
 
 
 # ---------------------------------------------------------------- CPU arms
