@@ -232,15 +232,16 @@ int wq3d_ocean_sound_speed_noalloc(const wq3d_ocean* ocean, double earth_radius,
 
 enum { WQ3D_CLASSIC_RAY = 0, WQ3D_HYBRID_GAUSSIAN = 1 }; /* wave_queue.h:90 */
 /* Arithmetic form.  WQ3D_FP64: the reference's FP64 arithmetic throughout.
- * WQ3D_FP32C: the same, with the CPA search's comparisons screened in FP32
- * and finished in FP64 where the screen cannot decide (the eigenrays equal
- * the FP64 arithmetic's bit for bit, so WQ3D_FP64 queues are searched the
- * same way, but in the bounds-checked build).  WQ3D_FP32: additionally the sound speed,
- * its gradient and the ray derivatives of every wave_front::update
- * (wave_front.cc:125-178) in FP32, at the altitude offset rho - R, while
- * positions, directions, travel time, the distance terms and the CPA
- * Taylor fit stay FP64; its error against the FP64 form is measured, not
- * zero.  The adjoint is refused for WQ3D_FP32. */
+ * WQ3D_FP32C: the same, with (ray, target) pairs that the CPA search cannot
+ * keep rejected by FP32 bounds and the rest decided in FP64: the same
+ * eigenrays bit for bit.  WQ3D_FP64 queues are therefore searched that way
+ * too; only the bounds-checked build compares every pair of theirs in FP64.
+ * WQ3D_FP32: additionally the sound speed, its gradient and the ray
+ * derivatives of every wave_front::update (wave_front.cc:125-178) in FP32,
+ * at the altitude offset rho - R, while positions, directions, travel time,
+ * the distance terms and the CPA Taylor fit stay FP64; its error against
+ * the FP64 form is measured, not zero.  The adjoint is refused for
+ * WQ3D_FP32. */
 enum { WQ3D_FP64 = 0, WQ3D_FP32C = 1, WQ3D_FP32 = 2 };
 
 typedef struct wq3d_queue_desc {

@@ -792,14 +792,11 @@ __device__ __forceinline__ void work_append(const QueueDev& q, int p, uint8_t ki
     }
 }
 
-/* shadow slot of a reflecting ray: prev, curr, next (17 doubles each), the
- * next front's attenuation and phase (nf each), and the three loss
- * tangents its bottom bounces add; counts in shadow_cnt */
-/* a shadow slot: prev, curr and next states (17 doubles each), the next
+/* the shadow slot of a reflecting ray: prev, curr and next states (17 doubles each), the next
  * front's attenuation and phase (nf each), the three loss tangents of the
  * step's bottom bounces, and the phases again as they are when the caustic
  * hand-off of the neighbour below shifted them by -pi/2 before the
- * reflection (nf) */
+ * reflection (nf); counts in shadow_cnt */
 __device__ __forceinline__ size_t shadow_stride(const QueueDev& q) { return 54 + 3 * (size_t)q.nf; }
 
 __device__ __forceinline__ void ray_to(double* dst, const RayS& y) {

@@ -37,9 +37,10 @@ struct CpaTargets {
 
 /* the clusters of the targets in the given order, and the sum of their
  * extents in metres */
-inline double make_clusters(const std::vector<double>& r, const std::vector<double>& th, const std::vector<double>& ph,
-                     const std::vector<double>& sn, const std::vector<uint8_t>& branch,
-                     const std::vector<uint32_t>& order, std::vector<TgtCluster>* out) {
+inline double make_clusters(const std::vector<double>& r, const std::vector<double>& th,
+                            const std::vector<double>& ph, const std::vector<double>& sn,
+                            const std::vector<uint8_t>& branch, const std::vector<uint32_t>& order,
+                            std::vector<TgtCluster>* out) {
     out->clear();
     double total = 0.0;
     for (size_t b = 0; b < order.size(); b += 32) {
@@ -79,8 +80,9 @@ inline double make_clusters(const std::vector<double>& r, const std::vector<doub
  * columns are already compact (1.5 of 32 clusters survive a warp's bounds on
  * the sloped workload, 3 along the curve), random targets are not (27 of 128
  * on the reverberation workload, 126 in their own order). */
-inline void cpa_targets(const std::vector<double>& r, const std::vector<double>& th, const std::vector<double>& ph,
-                 const std::vector<double>& sn, const std::vector<uint8_t>& branch, CpaTargets* o) {
+inline void cpa_targets(const std::vector<double>& r, const std::vector<double>& th,
+                        const std::vector<double>& ph, const std::vector<double>& sn,
+                        const std::vector<uint8_t>& branch, CpaTargets* o) {
     o->index.clear();
     double lo[3], hi[3];
     for (size_t t = 0; t < r.size(); ++t) {
