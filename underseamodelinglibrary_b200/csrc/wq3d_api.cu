@@ -917,8 +917,7 @@ struct wq3d_queue : QueueRt {
         /* eigenray candidates grow with the fan: one block per SM for small
          * fans, up to EIG_BLOCKS */
         const int eig_blocks = std::min(EIG_BLOCKS, std::max(148, (n + 255) / 256));
-        /* and so do the items of its CPA search */
-        const int item_blocks = std::min(CPA_ITEM_BLOCKS, std::max(148, (n + 255) / 256));
+        const int item_blocks = cpa_item_blocks(n, h.n_patch, h.nt, 148, CPA_ITEM_BLOCKS);
         if (timing) tail = false;
         auto cpa_launch = [&](int k, cudaStream_t st) {
             const int cgrid = std::max(1, (h.n_patch + CPA_WARPS - 1) / CPA_WARPS);
@@ -1954,9 +1953,7 @@ int wq3d_queue_create(const wq3d_ocean* ocean, const wq3d_queue_desc* d, wq3d_qu
         uint32_t* cand = nullptr;
         if ((rc = q->alloc(&cand, 2 * CAND_LISTS * (size_t)h.cap_cand))) return cleanup(rc);
         h.cand = cand;
-        /* items of the CPA search: a few per patch at most on the measured
-         * workloads; k_cpa decides those that find no room */
-        h.cap_item = (uint32_t)std::max<size_t>(4096, std::min<size_t>((size_t)1 << 20, 2 * n));
+        h.cap_item = (uint32_t)cpa_item_capacity(nde, naz, nt);
         if ((rc = q->alloc(&h.items, h.cap_item))) return cleanup(rc);
         if ((rc = q->alloc(&h.rec, h.cap_rec)) || (rc = q->alloc(&h.rec_inten, (size_t)h.cap_rec * nf)) ||
             (rc = q->alloc(&h.rec_phase, (size_t)h.cap_rec * nf)) || (rc = q->alloc(&h.refl, h.cap_refl)))

@@ -134,4 +134,33 @@ inline void cpa_targets(const std::vector<double>& r, const std::vector<double>&
     }
 }
 
+/* the most patches of 32 rays that a fan is cut into (cpa_patches) */
+inline size_t cpa_patch_bound(size_t nde, size_t naz) {
+    size_t most = 0;
+    for (int s = 0; s <= 5; ++s) {
+        const size_t rows = 32 >> s, cols = (size_t)1 << s;
+        most = std::max(most, ((nde + rows - 1) / rows) * ((naz + cols - 1) / cols));
+    }
+    return most;
+}
+
+/* Room for the search's items (a patch and a target whose 32 pairs the
+ * bounds leave).  A few a patch in fans whose rays lie close, and two a ray
+ * are room enough; but patches of a coarse fan span kilometres and keep most
+ * targets, so there is room for every patch and target up to 2^18.  (k_cpa
+ * decides those that find none, one after another: 69 x 8 rays and 1500
+ * targets took 137 us a step with room for 4096 items, 43 with room for all.) */
+inline size_t cpa_item_capacity(size_t nde, size_t naz, size_t nt) {
+    return std::max({(size_t)4096, std::min((size_t)1 << 20, 2 * nde * naz),
+                     std::min((size_t)1 << 18, cpa_patch_bound(nde, naz) * nt)});
+}
+
+/* Blocks of four warps for them: one per 256 rays as for the eigenrays, and
+ * at most 16 items a warp where 24 patches keep every target, which a coarse
+ * fan's do; the count is not known when the launch is made. */
+inline int cpa_item_blocks(size_t n, size_t patches, size_t nt, int least, int most) {
+    const size_t want = std::max({(size_t)least, (n + 255) / 256, std::min<size_t>(patches, 24) * nt / 64});
+    return (int)std::min<size_t>(want, (size_t)most);
+}
+
 }  // namespace wq3d
