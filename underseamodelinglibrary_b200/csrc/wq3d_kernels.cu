@@ -2118,6 +2118,27 @@ struct WarpBuild {
         return hit >= 0 || virt != 0;
     }
 
+    /* How many cells of a side the walk takes first: those whose widths the
+     * first pass made, or all 32 where a cell's terms (one a frequency) cost
+     * more than a second pass of widths, since most walks then go on beyond
+     * 15 cells.  Per launch, 15 against 32 cells: 203 and 181 us with 64
+     * frequencies on 383 x 7 rays, 197 and 189 with 32 on the reverberation
+     * workload; 140 and 147 with 64 on 83 x 17 rays, whose walks are short.
+     * With 8 or fewer (one group of EIG_FG) the shorter start is the faster. */
+    __device__ int first_cells(int made) const { return q->nf > EIG_FG ? 32 : made; }
+
+    /* widths of cells 0..ncell-1, lane k's by width(), but for the first
+     * "have" that are at "made" */
+    template <class F>
+    __device__ const double* cell_widths(int have, const double* made, int ncell, bool skip, F width) {
+        if (ncell <= have) return made;
+        const double x = lane < have ? made[lane] : lane < ncell && !skip ? width() : 0.0;
+        __syncwarp();
+        sw[lane] = x;
+        __syncwarp();
+        return sw;
+    }
+
     /* spreading_hybrid_gaussian.cc:124-258 */
     __device__ void intensity_de(int de0, int a, const double* offset, const double* distance) {
         const QueueDev& Q = *q;
@@ -2145,17 +2166,16 @@ struct WarpBuild {
         double cell_width = wl, cell_dist = L + wl;
         for (int d0 = de0 - 2, at = 1; d0 >= 0; at = 0) {
             const int d = d0 - lane;
-            const int ncell = min(at ? EIG_SIDE - 1 : 32, d0 + 1);
+            const int ncell = min(at ? first_cells(EIG_SIDE - 1) : 32, d0 + 1);
             bool virt = false;
             double nm = 0.0, nmv = 0.0;
             if (lane < ncell) {
                 virt = C.on_edge[(d + 1) * Q.naz + a] && C.on_edge[d * Q.naz + a];
                 nm = Q.norm_de[d];
                 nmv = Q.norm_de[d + 1];
-                if (!at && !virt) sw[lane] = width_de(d, a, -1);
             }
-            __syncwarp();
-            if (run_cells(ncell, sw + at, virt, nm, nmv, 1.0, cell_dist, cell_width, &stop)) break;
+            const double* w = cell_widths(at ? EIG_SIDE - 1 : 0, sw + 1, ncell, virt, [&] { return width_de(d, a, -1); });
+            if (run_cells(ncell, w, virt, nm, nmv, 1.0, cell_dist, cell_width, &stop)) break;
             d0 -= ncell;
         }
         /* upper D/E cells: de0+1 up to num_de-2 */
@@ -2164,17 +2184,16 @@ struct WarpBuild {
         const int size = Q.nde - 1;
         for (int d0 = de0 + 1, at = 1; d0 < size; at = 0) {
             const int d = d0 + lane;
-            const int ncell = min(at ? EIG_SIDE - 2 : 32, size - d0);
+            const int ncell = min(at ? first_cells(EIG_SIDE - 2) : 32, size - d0);
             bool virt = false;
             double nm = 0.0, nmv = 0.0;
             if (lane < ncell) {
                 virt = C.on_edge[(d + 1) * Q.naz + a] && C.on_edge[d * Q.naz + a];
                 nm = Q.norm_de[d];
                 nmv = Q.norm_de[d - 1];
-                if (!at && !virt) sw[lane] = width_de(d, a, -1);
             }
-            __syncwarp();
-            if (run_cells(ncell, at ? su + 1 : sw, virt, nm, nmv, -1.0, cell_dist, cell_width, &stop)) break;
+            const double* w = cell_widths(at ? EIG_SIDE - 2 : 0, su + 1, ncell, virt, [&] { return width_de(d, a, -1); });
+            if (run_cells(ncell, w, virt, nm, nmv, -1.0, cell_dist, cell_width, &stop)) break;
             d0 += ncell;
         }
     }
@@ -2210,7 +2229,7 @@ struct WarpBuild {
         int marked = -1; /* index (in walk order) of the last cell marked */
         bool done = false;
         for (int k0 = 0, at = 1; !done && k0 < max_az; at = 0) {
-            const int len = at ? EIG_SIDE - 1 : 32;
+            const int len = at ? first_cells(EIG_SIDE - 1) : 32;
             const int k = k0 + lane;
             int a = start - k;
             a = ((a % max_az) + max_az) % max_az;
@@ -2229,11 +2248,10 @@ struct WarpBuild {
                 ncell = __ffs(stopmask) - 1;
                 fk = __shfl_sync(0xffffffffu, kind, ncell);
             }
-            if (!at && lane < ncell) sw[lane] = width_az(d, a);
             const double nm = (lane < ncell) ? norm(a) : 0.0;
-            __syncwarp();
+            const double* w = cell_widths(at ? EIG_SIDE - 1 : 0, sw + 1, ncell, false, [&] { return width_az(d, a); });
             int kst = -1;
-            const bool brk = (ncell > 0) && run_cells(ncell, sw + at, false, nm, nm, 1.0, cell_dist, cell_width, &kst);
+            const bool brk = (ncell > 0) && run_cells(ncell, w, false, nm, nm, 1.0, cell_dist, cell_width, &kst);
             if (brk) {
                 marked = k0 + kst; /* the threshold stop happens on a marked cell */
                 done = true;
@@ -2251,7 +2269,7 @@ struct WarpBuild {
         cell_dist = L - wc;
         done = false;
         for (int k0 = 0, at = 1; !done && k0 < max_az; at = 0) {
-            const int len = at ? EIG_SIDE - 1 : 32;
+            const int len = at ? first_cells(EIG_SIDE - 1) : 32;
             const int k = k0 + lane;
             const int a = (az0 + 1 + k) % max_az;
             int kind = 0;
@@ -2271,11 +2289,10 @@ struct WarpBuild {
                 ncell = __ffs(stopmask) - 1;
                 done = true;
             }
-            if (!at && lane < ncell) sw[lane] = width_az(d, a);
             const double nm = (lane < ncell) ? norm(a) : 0.0;
-            __syncwarp();
+            const double* w = cell_widths(at ? EIG_SIDE - 1 : 0, su + 1, ncell, false, [&] { return width_az(d, a); });
             int kst = -1;
-            if (ncell > 0 && run_cells(ncell, at ? su + 1 : sw, false, nm, nm, -1.0, cell_dist, cell_width, &kst))
+            if (ncell > 0 && run_cells(ncell, w, false, nm, nm, -1.0, cell_dist, cell_width, &kst))
                 done = true;
             k0 += len;
         }
