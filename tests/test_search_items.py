@@ -18,7 +18,7 @@ int main() {
     size_t nde, naz, nt, patches;
     while (std::scanf("%zu %zu %zu %zu", &nde, &naz, &nt, &patches) == 4)
         std::printf("%zu %zu %d\n", wq3d::cpa_patch_bound(nde, naz), wq3d::cpa_item_capacity(nde, naz, nt),
-                    wq3d::cpa_item_blocks(nde * naz, patches, nt, 148, 592));
+                    wq3d::cpa_item_blocks(nde * naz, patches, nt, 148));
     return 0;
 }
 """
@@ -55,9 +55,11 @@ def test_room_and_warps(ask):
         assert bound == p
         assert 4096 <= room <= 1 << 20
         assert room >= min(p * nt, 1 << 18) and room >= min(2 * nde * naz, 1 << 20)
-        assert 148 <= blocks <= 592
+        assert 148 <= blocks <= 7 * 148
         # 16 items a warp, if 24 patches keep every target
-        assert blocks == 592 or 4 * 16 * (blocks + 1) >= min(p, 24) * nt
+        assert blocks == 7 * 148 or 4 * 16 * (blocks + 1) >= min(p, 24) * nt
+        # a dense fan with few targets has a block for 256 rays
+        assert 24 * nt > 64 * 148 or blocks == min(max(148, -(-nde * naz // 256)), 592)
 
 
 def test_fans_that_used_to_overflow(ask):

@@ -345,7 +345,7 @@ namespace {
  * rays throughout: 30 for 36 of 1024 (sloped workload, step 100), 52 for 123
  * of 4096 (reverberation workload), 10 for 34 of 100 (Munk workload).  The
  * steep bands, which keep the most, come first. */
-constexpr int CPA_PARTS = 8;
+constexpr int CPA_PARTS = 64;
 
 void cpa_patches(const std::vector<double>& de, const std::vector<double>& az, size_t nt,
                  std::vector<CpaPatch>* out) {
@@ -379,7 +379,8 @@ void cpa_patches(const std::vector<double>& de, const std::vector<double>& az, s
     }
     std::stable_sort(bands.begin(), bands.end(), [](const Band& x, const Band& y) { return x.steep > y.steep; });
     /* A fan with fewer patches than the GPU has room for (592 schedulers,
-     * four warps each) splits the clusters, four a share at least. */
+     * four warps each) splits the clusters, four a share at least: 9 x 8 rays
+     * and 10,000 targets, 82 us a step in 8 shares and 36 in 64. */
     const size_t ncl = (nt + 31) / 32;
     const size_t parts = std::max<size_t>(
         1, std::min({(size_t)CPA_PARTS, 4 * 592 / std::max<size_t>(patches, 1), ncl / 4}));
@@ -917,7 +918,7 @@ struct wq3d_queue : QueueRt {
         /* eigenray candidates grow with the fan: one block per SM for small
          * fans, up to EIG_BLOCKS */
         const int eig_blocks = std::min(EIG_BLOCKS, std::max(148, (n + 255) / 256));
-        const int item_blocks = cpa_item_blocks(n, h.n_patch, h.nt, 148, CPA_ITEM_BLOCKS);
+        const int item_blocks = cpa_item_blocks(n, h.n_patch, h.nt, 148);
         if (timing) tail = false;
         auto cpa_launch = [&](int k, cudaStream_t st) {
             const int cgrid = std::max(1, (h.n_patch + CPA_WARPS - 1) / CPA_WARPS);

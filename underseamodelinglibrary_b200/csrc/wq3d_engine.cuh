@@ -279,7 +279,6 @@ __global__ void k_volume(__grid_constant__ const QueueDev q, int k);
 __global__ void k_commit(__grid_constant__ const QueueDev q, int k);
 __global__ void k_cpa(__grid_constant__ const QueueDev q, int k);
 __global__ void k_cpa_items(__grid_constant__ const QueueDev q, int k);
-constexpr int CPA_ITEM_BLOCKS = 4 * 148; /* four warps each */
 /* k_eigenray blocks (4 warps each, one candidate per warp pair at a
  * time): four per SM, so a step's candidates usually all run at once */
 constexpr int EIG_BLOCKS = 4 * 148;

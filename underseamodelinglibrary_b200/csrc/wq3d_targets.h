@@ -155,12 +155,13 @@ inline size_t cpa_item_capacity(size_t nde, size_t naz, size_t nt) {
                      std::min((size_t)1 << 18, cpa_patch_bound(nde, naz) * nt)});
 }
 
-/* Blocks of four warps for them: one per 256 rays as for the eigenrays, and
- * at most 16 items a warp where 24 patches keep every target, which a coarse
- * fan's do; the count is not known when the launch is made. */
-inline int cpa_item_blocks(size_t n, size_t patches, size_t nt, int least, int most) {
-    const size_t want = std::max({(size_t)least, (n + 255) / 256, std::min<size_t>(patches, 24) * nt / 64});
-    return (int)std::min<size_t>(want, (size_t)most);
+/* Blocks of four warps for them: one per 256 rays as for the eigenrays, up to
+ * four an SM, and at most 16 items a warp where 24 patches keep every target,
+ * which a coarse fan's do, up to the seven an SM that are resident; the count
+ * is not known when the launch is made. */
+inline int cpa_item_blocks(size_t n, size_t patches, size_t nt, size_t sms) {
+    return (int)std::max({sms, std::min(4 * sms, (n + 255) / 256),
+                          std::min(7 * sms, std::min<size_t>(patches, 24) * nt / 64)});
 }
 
 }  // namespace wq3d
