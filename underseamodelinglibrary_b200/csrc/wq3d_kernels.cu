@@ -1926,8 +1926,9 @@ namespace {
  * test needs are those that the lowest frequency adds; and divisions are
  * branch-free.  Per launch, with the event timing's overhead: 29.7 -> 24.3 us
  * (Munk workload, one or two candidates a step), 65 -> 46 us (sloped
- * workload, 907 x 53 rays); 300 -> 315 us with 32 frequencies, whose sums
- * dominate. */
+ * workload, 907 x 53 rays); with more than EIG_FG frequencies, whose sums
+ * dominate, as before (first_cells), and with more candidates than the GPU
+ * holds 209 -> 227 us (49 x 32 rays, 1,660 eigenrays a step). */
 constexpr int EIG_FG = 8;    /* frequencies per pass of a walk chunk's Gaussian terms */
 constexpr int EIG_SIDE = 16; /* cells on a side whose widths the first pass forms     */
 
